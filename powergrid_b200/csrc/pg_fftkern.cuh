@@ -1,0 +1,464 @@
+// Kernels of the pruned oversampled FFT passes (pg_fftpass.cu), one set per
+// length n = R1 * R2 = 2N.  Each translation unit pg_fft_len*.cu instantiates
+// some lengths (FftOps) so that they compile in parallel.
+//
+// Each length-n transform is two register passes with one shared-memory
+// transpose between them (the four-step form).  Forward, with m = R2 m1 + m2
+// and k = k1 + R1 k2:
+//   X[k] = sum_m2 W_R2^(m2 k2) * W_n^(m2 k1) * sum_m1 W_R1^(m1 k1) x[m].
+// The zero padding leaves m in [n/4, 3n/4), which is m1 in [R1/4, 3 R1/4) for
+// every m2: half of the first pass's inputs are literal zeros.  The inverse
+// uses the split the other way round (m = R1 m1 + m2, k = k1 + R2 k2), so that
+// the crop k in [n/4, 3n/4) is k2 in [R1/4, 3 R1/4): half of the second pass's
+// outputs are never formed.  Both directions then store (forward) or load
+// (inverse) grid rows r + R1 q, q < R2 <= 32, per thread, so the support of a
+// thread's rows is one 32-bit word (pg_nufft.cuh, FftSupport).
+//
+// What bounds the passes is memory: in 3-D every grid line crosses HBM once
+// per pass.  Rows of 8 adjacent y cells (64 bytes, the support's unit) that no
+// sample of the segment touches are neither computed, stored, loaded nor
+// cleared.
+#pragma once
+
+#include <algorithm>
+
+#include "pg_fftdft.cuh"
+#include "pg_fftpass.cuh"
+
+namespace pg {
+
+// Strided lines of the batch's grids: grid b = c * L + l holds `slabs` sets of
+// lines (z slabs in the x pass, one set in the z pass).
+struct FftLines {
+  uint64_t in_stride, out_stride;   // elements between consecutive (grid, slab) sets
+  uint64_t rstride;                 // elements between a line's consecutive rows
+  int L, slabs;
+  const uint32_t* list;             // active groups: segment << 24 | group of 8 adjacent columns
+  int nlist;
+  const uint32_t* rows;             // support words [segment][group][R1], or null: every row
+  int ngroups;                      // groups per segment in `rows`
+  const float2* tw;                 // W_n^(k1 m2): [R1][R2], then transposed [R2][R1]
+};
+
+// Image lines of the batch (rows along y).
+struct FftRows {
+  int L, C, c0;                     // segments, coils of the batch, their first map
+  int cgroup;                       // coils per image, 0: one image
+  uint64_t image_stride, phase_stride;
+  const float2* S;                  // coil maps or null
+  const float2* E;                  // extra image factor or null
+  const float2* W;                  // Wo (forward) / WoH (inverse) or null
+  const float* deapf;
+  const uint32_t* rows;             // support words [segment][R1]
+  const float2* tw;
+  int split;                        // forward: blocks per coil; inverse: blocks per image
+};
+
+struct FftOps {
+  int n;
+  pg_status (*rows_fwd)(const NufftGeom& g, const FftRows& a, const float2* x, float2* P, cudaStream_t s);
+  pg_status (*cols_fwd)(const FftLines& a, uint64_t nsets, const float2* in, float2* out, cudaStream_t s);
+  pg_status (*cols_inv)(const FftLines& a, uint64_t nsets, float2* in, int clear, float2* out, cudaStream_t s);
+  // out: `split` partial images per image, or (split == 1) x itself
+  pg_status (*rows_inv)(const NufftGeom& g, const FftRows& a, int nimages, const float2* Q, int accumulate,
+                        float2* out, cudaStream_t s);
+  int rows_per_block;
+};
+
+namespace fftk {
+
+__host__ __device__ constexpr int imax(int a, int b) { return a > b ? a : b; }
+__host__ __device__ constexpr int imin(int a, int b) { return a < b ? a : b; }
+
+// Row kernels: 16 lines per block (8, or 4 at n = 1024, where a pass has more
+// than 16 threads per line), so that the 2-D sizes still give a few hundred
+// blocks and the transpose fits 48 KB.
+template <int R1, int R2>
+struct RowGeo {
+  static constexpr int n = R1 * R2;
+  static constexpr int RB = n >= 1024 ? 4 : imax(R1, R2) > 16 ? 8 : 16;
+  static constexpr int T = (RB * imax(R1, R2) + 31) / 32 * 32;
+};
+// Shared layout [row][k1 < RA][m2 < RBk]: odd m2 stride (the second pass's
+// threads, one k1 each, hit distinct banks), row stride = RBk (mod 16).
+template <int RA, int RBk>
+struct RowSm {
+  static constexpr int S2 = RBk | 1;
+  static constexpr int base = RA * S2;
+  static constexpr int RS = base + (((RBk - base) % 16) + 16) % 16;
+};
+// Line kernels: CB adjacent columns per block, shared layout [k1][m2][col];
+// with 8 columns and an even R the k1 stride is padded by one row of columns
+// so that the second pass's half-warps (two k1) hit distinct banks.
+template <int R1, int R2>
+struct ColGeo {
+  static constexpr int n = R1 * R2;
+  static constexpr int CB = n <= 64 ? 32 : n <= 256 ? 16 : 8;
+  static constexpr int T = imin(256, (CB * imax(R1, R2) + 31) / 32 * 32);
+  static constexpr int stride(int RBk) { return RBk * CB + (CB == 8 && RBk % 2 == 0 ? 8 : 0); }
+  static constexpr size_t smem_fwd = (size_t)R1 * stride(R2) * sizeof(float2);
+  static constexpr size_t smem_inv = (size_t)R2 * stride(R1) * sizeof(float2);
+};
+
+__device__ __forceinline__ int parity2(int a, int b) { return (a + b) & 1; }
+
+// Image lines (ix, iz) of one coil: pre-kernel values (coil map, shot phase,
+// deapodization, checkerboard sign) formed once and kept in registers, then
+// per segment of the block's share the phase Wo and the FFT along y of the
+// zero-padded line -> P[c * L + l][iz][ix][0..n), supported groups only.
+template <int R1, int R2>
+__global__ void __launch_bounds__((RowGeo<R1, R2>::T)) k_fft_fwd_rows(NufftGeom g, FftRows a,
+                                                                      const float2* __restrict__ x,
+                                                                      float2* __restrict__ P) {
+  pdl_wait();
+  using RG = RowGeo<R1, R2>;
+  using SM = RowSm<R1, R2>;
+  constexpr int n = RG::n, RB = RG::RB, H = R1 / 2;
+  __shared__ float2 sh[RB * SM::RS];
+  const int Nn = n / 2, nrows = g.Nx * g.Nz;
+  const uint64_t N = g.nimg();
+  const int cs = blockIdx.x % (a.C * a.split);   // coils fastest: they share the rows' segment phases in L2
+  const int c = cs / a.split, part = cs - c * a.split;
+  const int l0 = a.L * part / a.split, l1 = a.L * (part + 1) / a.split;
+  const int cg = a.c0 + c;
+  const int img = a.cgroup > 0 ? cg / a.cgroup : 0;
+  const int r0 = blockIdx.x / (a.C * a.split) * RB;
+  // first pass: thread (row, m2); second pass: thread (row, k1)
+  const int m2 = threadIdx.x % R2, ra = threadIdx.x / R2;
+  const int k1 = threadIdx.x % R1, rb = threadIdx.x / R1;
+  const bool in_a = ra < RB && r0 + ra < nrows, in_b = rb < RB && r0 + rb < nrows;
+  float2 u[H];
+  uint64_t p0 = 0;
+  if (in_a) {
+    const int rg = r0 + ra, ix = rg % g.Nx, iz = rg / g.Nx;
+    const int pxz = ix + g.pad_off[0] + iz + g.pad_off[2];
+    p0 = (uint64_t)m2 + (uint64_t)Nn * rg;
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const uint64_t p = p0 + R2 * h;
+      float2 v = x[(uint64_t)img * a.image_stride + p];
+      if (a.S) {
+        const float2 sv = a.S[(uint64_t)cg * N + p];
+        v = a.E ? cmul(v, cmul(sv, a.E[p])) : cmul(sv, v);
+      }
+      const float f = parity2(pxz, R2 * h + m2 + n / 4) ? -a.deapf[p] : a.deapf[p];
+      u[h] = make_float2(v.x * f, v.y * f);
+    }
+  }
+  const float2* W = a.W ? a.W + (uint64_t)img * a.phase_stride : nullptr;
+  for (int l = l0; l < l1; ++l) {
+    if (in_a) {
+      float2 v[R1];
+#pragma unroll
+      for (int m1 = 0; m1 < R1; ++m1) v[m1] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int h = 0; h < H; ++h) v[R1 / 4 + h] = W ? cmul(W[(uint64_t)l * N + p0 + R2 * h], u[h]) : u[h];
+      dft<R1>(v, false);
+      float2* d = sh + ra * SM::RS + m2;
+      d[0] = v[0];
+#pragma unroll
+      for (int q = 1; q < R1; ++q) d[q * SM::S2] = twiddle(v[q], a.tw[q * R2 + m2], false);
+    }
+    __syncthreads();
+    if (in_b) {
+      const uint32_t sup = a.rows[l * R1 + k1];
+      float2 v[R2];
+      const float2* s = sh + rb * SM::RS + k1 * SM::S2;
+#pragma unroll
+      for (int q = 0; q < R2; ++q) v[q] = s[q];
+      dft<R2>(v, false);
+      float2* o = P + (((uint64_t)c * a.L + l) * nrows + r0 + rb) * n + k1;
+#pragma unroll
+      for (int k2 = 0; k2 < R2; ++k2)
+        if (sup >> k2 & 1u) o[R1 * k2] = v[k2];
+    }
+    __syncthreads();
+  }
+}
+
+// Strided lines forward: per active column the n/2 nonzero rows, zero padded
+// to n, FFT along the line -> the output's supported rows.
+template <int R1, int R2>
+__global__ void __launch_bounds__((ColGeo<R1, R2>::T)) k_fft_fwd_cols(FftLines a, uint64_t set0,
+                                                                      const float2* __restrict__ in,
+                                                                      float2* __restrict__ out) {
+  pdl_wait();
+  using CG = ColGeo<R1, R2>;
+  constexpr int CB = CG::CB, T = CG::T, S1 = CG::stride(R2), H = R1 / 2;
+  extern __shared__ float2 sh[];
+  const uint64_t y = set0 + blockIdx.y;      // coil * slabs + slab
+  const uint64_t c = y / a.slabs, slab = y - c * a.slabs;
+  const int e0 = blockIdx.x * (CB / 8);
+#pragma unroll
+  for (int it0 = 0; it0 < CB * R2; it0 += T) {
+    const int it = it0 + threadIdx.x;
+    if ((CB * R2) % T != 0 && it >= CB * R2) break;
+    const int col = it % CB, m2 = it / CB;
+    const int e = e0 + col / 8;
+    if (e >= a.nlist) continue;
+    const uint32_t ent = a.list[e];
+    const float2* s = in + ((c * a.L + (ent >> 24)) * a.slabs + slab) * a.in_stride + (uint64_t)(ent & 0xffffffu) * 8 +
+                      (col & 7) + (uint64_t)m2 * a.rstride;
+    float2 v[R1];
+#pragma unroll
+    for (int m1 = 0; m1 < R1; ++m1) v[m1] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int h = 0; h < H; ++h) v[R1 / 4 + h] = s[(uint64_t)(R2 * h) * a.rstride];
+    dft<R1>(v, false);
+    float2* d = sh + m2 * CB + col;
+    d[0] = v[0];
+#pragma unroll
+    for (int q = 1; q < R1; ++q) d[q * S1] = twiddle(v[q], a.tw[q * R2 + m2], false);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it0 = 0; it0 < CB * R1; it0 += T) {
+    const int it = it0 + threadIdx.x;
+    if ((CB * R1) % T != 0 && it >= CB * R1) break;
+    const int col = it % CB, k1 = it / CB;
+    const int e = e0 + col / 8;
+    if (e >= a.nlist) continue;
+    const uint32_t ent = a.list[e];
+    const uint32_t l = ent >> 24, grp = ent & 0xffffffu;
+    const uint32_t sup = a.rows ? a.rows[((uint64_t)l * a.ngroups + grp) * R1 + k1] : 0xffffffffu;
+    float2 u[R2];
+    const float2* s = sh + k1 * S1 + col;
+#pragma unroll
+    for (int q = 0; q < R2; ++q) u[q] = s[q * CB];
+    dft<R2>(u, false);
+    float2* o = out + ((c * a.L + l) * a.slabs + slab) * a.out_stride + (uint64_t)grp * 8 + (col & 7) +
+                (uint64_t)k1 * a.rstride;
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2)
+      if (sup >> k2 & 1u) o[(uint64_t)(R1 * k2) * a.rstride] = u[k2];
+  }
+}
+
+// Strided lines inverse: per active column the supported rows (the others are
+// zero), inverse FFT along the line, the n/2 cropped rows -> output.  Every
+// supported cell is read exactly once; with CLEAR it is zeroed after that read
+// (through inw, the same grids), which leaves the grids zero for the next
+// adjoint spread.
+template <int R1, int R2, bool CLEAR>
+__global__ void __launch_bounds__((ColGeo<R1, R2>::T)) k_fft_inv_cols(FftLines a, uint64_t set0,
+                                                                      const float2* __restrict__ in, float2* inw,
+                                                                      float2* __restrict__ out) {
+  pdl_wait();
+  using CG = ColGeo<R1, R2>;
+  constexpr int CB = CG::CB, T = CG::T, S1 = CG::stride(R1), H = R1 / 2;
+  extern __shared__ float2 sh[];
+  const uint64_t y = set0 + blockIdx.y;
+  const uint64_t c = y / a.slabs, slab = y - c * a.slabs;
+  const int e0 = blockIdx.x * (CB / 8);
+  const float2* tw = a.tw + R1 * R2;       // transposed: [k1 < R2][m2 < R1]
+#pragma unroll
+  for (int it0 = 0; it0 < CB * R1; it0 += T) {
+    const int it = it0 + threadIdx.x;
+    if ((CB * R1) % T != 0 && it >= CB * R1) break;
+    const int col = it % CB, m2 = it / CB;
+    const int e = e0 + col / 8;
+    if (e >= a.nlist) continue;
+    const uint32_t ent = a.list[e];
+    const uint32_t l = ent >> 24, grp = ent & 0xffffffu;
+    const uint32_t sup = a.rows ? a.rows[((uint64_t)l * a.ngroups + grp) * R1 + m2] : 0xffffffffu;
+    const uint64_t o = ((c * a.L + l) * a.slabs + slab) * a.in_stride + (uint64_t)grp * 8 + (col & 7) +
+                       (uint64_t)m2 * a.rstride;
+    float2 v[R2];
+#pragma unroll
+    for (int m1 = 0; m1 < R2; ++m1) {
+      v[m1] = make_float2(0.f, 0.f);
+      if (sup >> m1 & 1u) {
+        if constexpr (CLEAR) v[m1] = inw[o + (uint64_t)(R1 * m1) * a.rstride];
+        else v[m1] = in[o + (uint64_t)(R1 * m1) * a.rstride];
+      }
+    }
+    dft<R2>(v, true);
+    float2* d = sh + m2 * CB + col;
+    d[0] = v[0];
+#pragma unroll
+    for (int q = 1; q < R2; ++q) d[q * S1] = twiddle(v[q], tw[q * R1 + m2], true);
+    if constexpr (CLEAR) {
+#pragma unroll
+      for (int m1 = 0; m1 < R2; ++m1)
+        if (sup >> m1 & 1u) inw[o + (uint64_t)(R1 * m1) * a.rstride] = make_float2(0.f, 0.f);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it0 = 0; it0 < CB * R2; it0 += T) {
+    const int it = it0 + threadIdx.x;
+    if ((CB * R2) % T != 0 && it >= CB * R2) break;
+    const int col = it % CB, k1 = it / CB;
+    const int e = e0 + col / 8;
+    if (e >= a.nlist) continue;
+    const uint32_t ent = a.list[e];
+    float2 u[R1];
+    const float2* s = sh + k1 * S1 + col;
+#pragma unroll
+    for (int q = 0; q < R1; ++q) u[q] = s[q * CB];
+    dft<R1>(u, true);
+    float2* o = out + ((c * a.L + (ent >> 24)) * a.slabs + slab) * a.out_stride + (uint64_t)(ent & 0xffffffu) * 8 +
+                (col & 7) + (uint64_t)k1 * a.rstride;
+#pragma unroll
+    for (int h = 0; h < H; ++h) o[(uint64_t)(R2 * h) * a.rstride] = u[R1 / 4 + h];
+  }
+}
+
+// Last inverse pass: lines (ix, iz) of the block's share of an image's grids,
+// inverse FFT along y, crop, WoH, conj coil map and conj shot phase, summed
+// over the share in grid order in registers; deapodization and sign once at
+// the end.  One partial image per share (or the image itself for one share):
+// the grids' images never reach memory.
+template <int R1, int R2>
+__global__ void __launch_bounds__((RowGeo<R1, R2>::T)) k_fft_inv_rows(NufftGeom g, FftRows a, int nimages,
+                                                                      const float2* __restrict__ Q, int accumulate,
+                                                                      float2* __restrict__ out) {
+  pdl_wait();
+  using RG = RowGeo<R1, R2>;
+  using SM = RowSm<R2, R1>;
+  constexpr int n = RG::n, RB = RG::RB, H = R1 / 2;
+  __shared__ float2 sh[RB * SM::RS];
+  const int Nn = n / 2, nrows = g.Nx * g.Nz;
+  const uint64_t N = g.nimg();
+  const int is = blockIdx.x % (nimages * a.split);
+  const int i = is / a.split, part = is - i * a.split;
+  // the image's coils inside the batch [c0, c0 + C)
+  const int img = a.cgroup > 0 ? a.c0 / a.cgroup + i : 0;
+  const int ca = a.cgroup > 0 ? max(a.c0, img * a.cgroup) : a.c0;
+  const int cb = a.cgroup > 0 ? min(a.c0 + a.C, (img + 1) * a.cgroup) : a.c0 + a.C;
+  const int nb = (cb - ca) * a.L;
+  const int b0 = (int)((int64_t)nb * part / a.split), b1 = (int)((int64_t)nb * (part + 1) / a.split);
+  const int r0 = blockIdx.x / (nimages * a.split) * RB;
+  // first pass: thread (row, m2 < R1); second pass: thread (row, k1 < R2)
+  const int m2 = threadIdx.x % R1, ra = threadIdx.x / R1;
+  const int k1 = threadIdx.x % R2, rb = threadIdx.x / R2;
+  const bool in_a = ra < RB && r0 + ra < nrows, in_b = rb < RB && r0 + rb < nrows;
+  const uint64_t p0 = (uint64_t)k1 + (uint64_t)Nn * (r0 + rb);
+  const float2* W = a.W ? a.W + (uint64_t)img * a.phase_stride : nullptr;
+  const float2* tw = a.tw + n;             // transposed: [k1 < R2][m2 < R1]
+  float2 acc[H], coil[H];                  // over the share; over the current coil's segments
+#pragma unroll
+  for (int h = 0; h < H; ++h) acc[h] = coil[h] = make_float2(0.f, 0.f);
+  for (int b = b0; b < b1; ++b) {
+    const int c = ca + b / a.L, l = b % a.L;
+    if (in_a) {
+      const uint32_t sup = a.rows[l * R1 + m2];
+      const float2* s = Q + (((uint64_t)(c - a.c0) * a.L + l) * nrows + r0 + ra) * n + m2;
+      float2 v[R2];
+#pragma unroll
+      for (int m1 = 0; m1 < R2; ++m1) {
+        v[m1] = make_float2(0.f, 0.f);
+        if (sup >> m1 & 1u) v[m1] = s[R1 * m1];
+      }
+      dft<R2>(v, true);
+      float2* d = sh + ra * SM::RS + m2;
+      d[0] = v[0];
+#pragma unroll
+      for (int q = 1; q < R2; ++q) d[q * SM::S2] = twiddle(v[q], tw[q * R1 + m2], true);
+    }
+    __syncthreads();
+    if (in_b) {
+      float2 u[R1];
+      const float2* s = sh + rb * SM::RS + k1 * SM::S2;
+#pragma unroll
+      for (int q = 0; q < R1; ++q) u[q] = s[q];
+      dft<R1>(u, true);
+      const bool last = l == a.L - 1 || b == b1 - 1;   // the coil's last segment here
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        float2 v = u[R1 / 4 + h];
+        if (W) v = cmul(v, W[(uint64_t)l * N + p0 + R2 * h]);
+        coil[h] = cadd(coil[h], v);
+      }
+      if (last) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          float2 v = coil[h];
+          if (a.S) {
+            const float2 sv = cconj(a.S[(uint64_t)c * N + p0 + R2 * h]);
+            v = a.E ? cmul(cmul(sv, cconj(a.E[p0 + R2 * h])), v) : cmul(v, sv);
+          }
+          acc[h] = cadd(acc[h], v);
+          coil[h] = make_float2(0.f, 0.f);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (!in_b) return;
+  const int rg = r0 + rb, ix = rg % g.Nx, iz = rg / g.Nx;
+  const int pxz = ix + g.crop_off[0] + iz + g.crop_off[2];
+  const bool add = a.split == 1 && (accumulate || (a.cgroup > 0 && img * a.cgroup < a.c0));
+  float2* o = a.split == 1 ? out + (uint64_t)img * a.image_stride : out + (uint64_t)is * N;
+#pragma unroll
+  for (int h = 0; h < H; ++h) {
+    const uint64_t p = p0 + R2 * h;
+    const float f = parity2(pxz, R2 * h + k1 + n / 4) ? -a.deapf[p] : a.deapf[p];
+    const float2 v = make_float2(acc[h].x * f, acc[h].y * f);
+    o[p] = add ? cadd(o[p], v) : v;
+  }
+}
+
+template <typename K>
+pg_status allow_smem(K kernel, size_t bytes) {
+  if (bytes > 48 * 1024) PG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  return PG_OK;
+}
+
+constexpr uint64_t kMaxGridY = 65535;
+
+template <int R1, int R2>
+pg_status rows_fwd(const NufftGeom& g, const FftRows& a, const float2* x, float2* P, cudaStream_t s) {
+  using RG = RowGeo<R1, R2>;
+  PG_LAUNCH_PDL((k_fft_fwd_rows<R1, R2>), (unsigned)(a.C * a.split) * ceil_div((uint64_t)g.Nx * g.Nz, RG::RB),
+                RG::T, 0, s, g, a, x, P);
+  return PG_OK;
+}
+
+template <int R1, int R2>
+pg_status rows_inv(const NufftGeom& g, const FftRows& a, int nimages, const float2* Q, int accumulate, float2* out,
+                   cudaStream_t s) {
+  using RG = RowGeo<R1, R2>;
+  PG_LAUNCH_PDL((k_fft_inv_rows<R1, R2>), (unsigned)(nimages * a.split) * ceil_div((uint64_t)g.Nx * g.Nz, RG::RB),
+                RG::T, 0, s, g, a, nimages, Q, accumulate, out);
+  return PG_OK;
+}
+
+template <int R1, int R2>
+pg_status cols_fwd(const FftLines& a, uint64_t nsets, const float2* in, float2* out, cudaStream_t s) {
+  using CG = ColGeo<R1, R2>;
+  if (a.nlist == 0) return PG_OK;
+  PG_TRY(allow_smem(k_fft_fwd_cols<R1, R2>, CG::smem_fwd));
+  for (uint64_t s0 = 0; s0 < nsets; s0 += kMaxGridY)
+    PG_LAUNCH_PDL((k_fft_fwd_cols<R1, R2>), dim3(ceil_div(a.nlist, CG::CB / 8), (unsigned)std::min(kMaxGridY, nsets - s0)),
+                  CG::T, CG::smem_fwd, s, a, s0, in, out);
+  return PG_OK;
+}
+
+template <int R1, int R2>
+pg_status cols_inv(const FftLines& a, uint64_t nsets, float2* in, int clear, float2* out, cudaStream_t s) {
+  using CG = ColGeo<R1, R2>;
+  if (a.nlist == 0) return PG_OK;
+  PG_TRY(clear ? allow_smem(k_fft_inv_cols<R1, R2, true>, CG::smem_inv)
+               : allow_smem(k_fft_inv_cols<R1, R2, false>, CG::smem_inv));
+  for (uint64_t s0 = 0; s0 < nsets; s0 += kMaxGridY) {
+    const dim3 grid(ceil_div(a.nlist, CG::CB / 8), (unsigned)std::min(kMaxGridY, nsets - s0));
+    if (clear)
+      PG_LAUNCH_PDL((k_fft_inv_cols<R1, R2, true>), grid, CG::T, CG::smem_inv, s, a, s0, (const float2*)in, in, out);
+    else
+      PG_LAUNCH_PDL((k_fft_inv_cols<R1, R2, false>), grid, CG::T, CG::smem_inv, s, a, s0, (const float2*)in,
+                    (float2*)nullptr, out);
+  }
+  return PG_OK;
+}
+
+}  // namespace fftk
+
+template <int R1, int R2>
+const FftOps* fft_ops() {
+  static const FftOps ops{R1 * R2, fftk::rows_fwd<R1, R2>, fftk::cols_fwd<R1, R2>, fftk::cols_inv<R1, R2>,
+                          fftk::rows_inv<R1, R2>, fftk::RowGeo<R1, R2>::RB};
+  return &ops;
+}
+
+}  // namespace pg

@@ -21,7 +21,8 @@
 //     (segment window, tile)); the adjoint spreads each bin into a padded
 //     shared-memory tile and flushes the tile once, so global atomics are
 //     per tile cell, not per tap;
-//   * cuFFT runs only the oversampled FFT, batched over coils x segments.
+//   * the oversampled FFT is pruned passes of our own for N a multiple of 8
+//     (pg_fftpass.cu); cuFFT, batched over coils x segments, for other sizes.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -1078,7 +1079,10 @@ pg_status nufft_plan_create(std::unique_ptr<NufftPlan>* out, uint64_t M, float g
   PG_TRY(p->lut.upload(lut.data(), lut.size(), s));
   p->lut_max = *std::max_element(lut.begin(), lut.end());
   PG_TRY(p->deap.upload(deap.data(), deap.size(), s));
-  // power-of-two 2N grids run the pruned, fused FFT passes; PG_CUFFT=1 keeps cuFFT
+  // 2N grids with N a multiple of 8 run the pruned, fused FFT passes: 1.5-1.7x
+  // cuFFT's time per operator pair at N = 96 and 208 (pg_fftpass.cu).  Other N
+  // keep cuFFT: the passes' groups of 8 cells and radix-16 pass need 16 | 2N.
+  // PG_CUFFT=1 keeps cuFFT everywhere.
   {
     const char* e = getenv("PG_CUFFT");
     p->own_fft = fftpass_supported(g) && !(e && e[0] == '1');
@@ -1138,6 +1142,12 @@ std::unique_ptr<Binning> binning_share(const Binning& b) {
   o->l0.borrow(b.l0);
   o->aa.borrow(b.aa);
   o->subprob.borrow(b.subprob);
+  o->sup.ylist.borrow(b.sup.ylist);
+  o->sup.xylist.borrow(b.sup.xylist);
+  o->sup.ymask.borrow(b.sup.ymask);
+  o->sup.xmask.borrow(b.sup.xmask);
+  o->sup.ny = b.sup.ny;
+  o->sup.nxy = b.sup.nxy;
   return o;
 }
 
@@ -1169,6 +1179,9 @@ pg_status nufft_build_binning(NufftPlan* p, int L, int K, const int* l0_host, co
   if (l0_host) PG_TRY(l0d.upload(l0_host, M, s));
   PG_LAUNCH(k_prepare, ceil_div(M, 256), 256, 0, s, g, M, p->kx.p, p->ky.p, p->kz.p, p->lut.p, t,
             l0_host ? l0d.p : nullptr, st_o.p, wxy_o.p, g.dim == 3 ? wz_o.p : nullptr, key.p);
+
+  if (p->own_fft)
+    PG_TRY(fftpass_support(g, M, L, K, st_o.p, l0_host ? l0d.p : nullptr, &b->sup, s));
 
   // Stable counting sort by key on the device (bit-exact against a CPU one).
   DevBuf<uint32_t> starts_d;
@@ -1577,20 +1590,8 @@ pg_status nufft_forward(NufftPlan* p, const NufftBatch& b, const float2* x, floa
       PG_TRY(ensure_workspace(p, B, nullptr, s));
       PG_TRY(grow(p->work->fin, fftpass_scratch(g, B), s));
       ProfScope ps("fft_fwd", s);
-      if (b.cgroup > 0) {
-        // one pass per image over its coils of the batch, into their grids
-        for (int i0 = c0; i0 < c0 + nb;) {
-          const int img = i0 / b.cgroup;
-          const int i1 = std::min(c0 + nb, (img + 1) * b.cgroup);
-          PG_TRY(fftpass_forward(g, (i1 - i0) * L, L, x + (uint64_t)img * b.image_stride, b.S, i0, b.E,
-                                 b.Wo ? b.Wo + (uint64_t)img * b.phase_stride : nullptr, p->deapf.p, p->tw2d.p,
-                                 p->work->fin.p, p->work->grids.p + (uint64_t)(i0 - c0) * L * G, s));
-          i0 = i1;
-        }
-      } else {
-        PG_TRY(fftpass_forward(g, B, L, x, b.S, c0, b.E, b.Wo, p->deapf.p, p->tw2d.p, p->work->fin.p,
-                               p->work->grids.p, s));
-      }
+      const FftBatch fb{nb, L, c0, b.S, b.E, b.cgroup, b.image_stride, b.phase_stride};
+      PG_TRY(fftpass_forward(g, fb, bin->sup, x, b.Wo, p->deapf.p, p->tw2d.p, p->work->fin.p, p->work->grids.p, s));
     } else {
     cufftHandle h;
     PG_TRY(ensure_workspace(p, B, &h, s));
@@ -1693,8 +1694,10 @@ pg_status nufft_adjoint(NufftPlan* p, const NufftBatch& b, const float2* y, floa
     PG_TRY(grow(p->work->vs, (uint64_t)nb * bin->M * K, s));
     {
       ProfScope ps("prep", s);
-      // a self-clearing target is already zero: only the values are formed
-      const uint64_t n4 = self_clear ? 0 : (uint64_t)B * G / 2;   // G is even: float2 pairs -> float4 words
+      // a self-clearing target is already zero, and the own 3-D passes read
+      // only the supported cells: only cuFFT needs every cell cleared
+      if (p->own_fft && !self_clear) PG_TRY(fftpass_clear(g, FftBatch{nb, L}, bin->sup, target, s));
+      const uint64_t n4 = p->own_fft ? 0 : (uint64_t)B * G / 2;   // G is even: float2 pairs -> float4 words
       const uint64_t work = std::max<uint64_t>(n4, bin->M);
       PG_LAUNCH(k_adjoint_prep, (unsigned)std::min<uint64_t>(ceil_div(work, 256), 8ull * sm_count()), 256, 0, s, n4,
                 reinterpret_cast<float4*>(target), nb, bin->M, K, bin->perm.p, aa, yc, b.data_stride,
@@ -1718,24 +1721,13 @@ pg_status nufft_adjoint(NufftPlan* p, const NufftBatch& b, const float2* y, floa
     const int acc = (b.accumulate || c0 > 0) ? 1 : 0;
     if (p->own_fft) {
       PG_TRY(grow(p->work->fin, fftpass_scratch(g, B), s));
-      PG_TRY(grow(p->work->rimg, (uint64_t)B * g.nimg(), s));
+      const FftBatch fb{nb, L, c0, b.S, b.E, b.cgroup, b.image_stride, b.phase_stride};
+      const int nimages = b.cgroup > 0 ? (c0 + nb - 1) / b.cgroup - c0 / b.cgroup + 1 : 1;
+      const int parts = fftpass_partials(g, fb, nimages);
+      if (parts > 1) PG_TRY(grow(p->work->rimg, (uint64_t)parts * nimages * g.nimg(), s));
       ProfScope ps("fft_adj", s);
-      if (b.cgroup > 0) {
-        // one pass per image over its coils of the batch; an image whose
-        // coils began in an earlier batch adds to its sum
-        for (int i0 = c0; i0 < c0 + nb;) {
-          const int img = i0 / b.cgroup;
-          const int i1 = std::min(c0 + nb, (img + 1) * b.cgroup);
-          const int acc_img = (b.accumulate || i0 > img * b.cgroup) ? 1 : 0;
-          PG_TRY(fftpass_adjoint(g, (i1 - i0) * L, L, target + (uint64_t)(i0 - c0) * L * G, self_clear, b.S, i0, b.E,
-                                 b.WoH ? b.WoH + (uint64_t)img * b.phase_stride : nullptr, p->deapf.p, p->tw2d.p,
-                                 p->work->fin.p, p->work->rimg.p, acc_img, x + (uint64_t)img * b.image_stride, s));
-          i0 = i1;
-        }
-      } else {
-        PG_TRY(fftpass_adjoint(g, B, L, target, self_clear, b.S, c0, b.E, b.WoH, p->deapf.p, p->tw2d.p,
-                               p->work->fin.p, p->work->rimg.p, acc, x, s));
-      }
+      PG_TRY(fftpass_adjoint(g, fb, bin->sup, target, self_clear, b.WoH, p->deapf.p, p->tw2d.p, p->work->fin.p,
+                             p->work->rimg.p, acc, x, s));
       if (self_clear) p->work->agrids_clean = true;   // the first inverse pass leaves the target zero
       continue;
     }

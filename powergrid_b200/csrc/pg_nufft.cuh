@@ -44,6 +44,17 @@ struct NufftTune {
   static NufftTune defaults();
 };
 
+// Grid cells that a segmentation's taps reach, in groups of 8 adjacent y
+// cells (pg_fftpass.cu).  The own FFT passes leave every other cell alone.
+struct FftSupport {
+  DevBuf<uint32_t> ylist;    // segment << 24 | y group, with a tap at any x (ny entries)
+  DevBuf<uint32_t> xylist;   // segment << 24 | x * (Gy / 8) + y group (3-D, nxy entries)
+  // support words of a thread's grid rows r + R1 q, bit q: [segment][R1] along
+  // y, [segment][y group][R1] along x
+  DevBuf<uint32_t> ymask, xmask;
+  int ny = 0, nxy = 0;
+};
+
 // Per-(trajectory, segmentation) sample binning used by both directions.
 // All per-sample arrays are in sorted order (stable by bin key).
 struct Binning {
@@ -59,6 +70,7 @@ struct Binning {
   DevBuf<float2> aa;         // K per sample: interpolator values AA(m, l0..l0+K-1)
   DevBuf<int4> subprob;      // (tile index, l0, first sorted sample, count)
   DevBuf<uint32_t> keys;     // bin key per original sample
+  FftSupport sup;            // for the own FFT passes
   int nsub = 0;
   int submax = 0;            // most samples in one subproblem
   uint64_t nkeys = 0;
@@ -77,7 +89,7 @@ struct NufftWork {
   bool agrids_clean = false;
   DevBuf<float2> fin;       // forward FFT input; its zero-pad border stays zero
   DevBuf<float2> vs;        // adjoint: per-sample segment values in binned order
-  DevBuf<float2> rimg;      // adjoint with the plan's own FFT passes: one image per grid
+  DevBuf<float2> rimg;      // adjoint with the plan's own FFT passes: partial images
   DevBuf<unsigned> queue;   // work-queue words of the persistent spread launches
   DevBuf<char> fft_work;
 };
@@ -91,7 +103,7 @@ struct NufftPlan {
   float lut_max = 0.f;           // largest per-axis tap weight
   DevBuf<float> deap;            // Nx + Ny + Nz reciprocal-transform factors
   DevBuf<float> deapf;           // per voxel 1/(OS^d k), 0 where k is NaN
-  bool own_fft = false;          // pruned fused 2-D FFT passes instead of cuFFT
+  bool own_fft = false;          // pruned fused FFT passes instead of cuFFT
   DevBuf<float2> tw2d;           // their twiddle table
   std::unique_ptr<Binning> plain;  // binning without segmentation (L = 1)
   // grid workspace (possibly shared) and cuFFT plans, keyed by batch size

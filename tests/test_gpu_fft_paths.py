@@ -72,6 +72,35 @@ def test_own_fft_passes_match_cufft(pg, n):
     assert e_f <= FORMS_TOL and e_a <= FORMS_TOL
 
 
+@pytest.mark.parametrize("n", list(range(8, 257, 8)) + [512])
+def test_own_fft_passes_every_length(pg, n):
+    """Every supported length 2n (each has its own factorisation), with and
+    without segments: their supports differ, and the second adjoint of a plan
+    finds the grids as the first one left them."""
+    from powergrid_b200 import synthetic as S
+    arrays, own = _ts_sense(pg, n, 4096, 3, 2, 90 + n)
+    _, ref = _cufft_form(lambda: _ts_sense(pg, n, 4096, 3, 2, 90 + n))
+    x = S.image(S.Rng(7), n * n)
+    for a, b in ((own[2], ref[2]), (own[0], ref[0])):
+        y = b * x
+        assert rel_l2(a * x, y) <= FORMS_TOL
+        for _ in range(2):
+            assert rel_l2(a / y, b / y) <= FORMS_TOL
+
+
+@pytest.mark.parametrize("n,nz,L", [(24, 24, 1), (40, 56, 3), (104, 8, 5), (48, 24, 12)])
+def test_own_fft_passes_3d_odd_factors(pg, n, nz, L):
+    """3-D with lengths that are no powers of two, one segment and many."""
+    from powergrid_b200 import synthetic as S
+    _, own = _ts_sense(pg, n, 600, L, 3, 50 + n, nz=nz)
+    _, ref = _cufft_form(lambda: _ts_sense(pg, n, 600, L, 3, 50 + n, nz=nz))
+    x = S.image(S.Rng(9), n * n * nz)
+    y = ref[2] * x
+    assert rel_l2(own[2] * x, y) <= FORMS_TOL
+    for _ in range(2):
+        assert rel_l2(own[2] / y, ref[2] / y) <= FORMS_TOL
+
+
 @pytest.mark.parametrize("L,nc", [(1, 1), (4, 3), (8, 8)])
 def test_fused_cluster_passes_equal_separate_passes(pg, L, nc):
     """The 256x256 grids' one-launch cluster form (rows in each CTA's shared
