@@ -102,12 +102,14 @@ void kb_table(float gridos, std::vector<float>* lut, float* beta_out) {
 // float sequence with no contraction, so the LUT entry chosen is identical.
 // A window has 9 cells only when s is an integer, and then both end cells
 // sit at distance W/2 and weigh 0; the nonzero taps therefore always fit in
-// 8 consecutive cells starting at `st`.  Cells outside [lo, hi] weigh 0.
-__device__ __forceinline__ int axis_taps(float k, int n_img, float os, float kw, const float* __restrict__ lut,
+// 8 consecutive cells starting at `st`.  Cells outside [lo, hi] weigh 0.  A
+// window past the grid's end (k up to 1.05 N/2 is accepted) is empty; its start
+// stays inside the grid, so that every sample has a tile.
+__device__ __forceinline__ int axis_taps(float k, int n_img, int g_cells, float os, float kw, const float* __restrict__ lut,
                                          int nlut, float* w) {
   int lo, hi;
   const float s = kb_window(k, n_img, os, kw, &lo, &hi);
-  const int st = (hi - lo == 8) ? lo + 1 : lo;
+  const int st = min((hi - lo == 8) ? lo + 1 : lo, g_cells - 1);
   const float kw2 = __fmul_rn(kw, kw);
 #pragma unroll
   for (int a = 0; a < 8; ++a) {
@@ -135,15 +137,15 @@ __global__ void k_prepare(NufftGeom g, uint64_t M, const float* __restrict__ kx,
   if (i >= M) return;
   float w[8];
   const float c = g.sign_c;
-  const int sx = axis_taps(kx[i], g.Nx, g.os, g.kw, lut, g.nlut, w);
+  const int sx = axis_taps(kx[i], g.Nx, g.Gx, g.os, g.kw, lut, g.nlut, w);
 #pragma unroll
   for (int a = 0; a < 8; ++a) wxy[i * 16 + a] = ((sx + a) & 1) ? -c * w[a] : c * w[a];
-  const int sy = axis_taps(ky[i], g.Ny, g.os, g.kw, lut, g.nlut, w);
+  const int sy = axis_taps(ky[i], g.Ny, g.Gy, g.os, g.kw, lut, g.nlut, w);
 #pragma unroll
   for (int a = 0; a < 8; ++a) wxy[i * 16 + 8 + a] = ((sy + a) & 1) ? -w[a] : w[a];
   int sz = 0;
   if (g.dim == 3) {
-    sz = axis_taps(kz[i], g.Nz, g.os, g.kw, lut, g.nlut, w);
+    sz = axis_taps(kz[i], g.Nz, g.Gz, g.os, g.kw, lut, g.nlut, w);
 #pragma unroll
     for (int a = 0; a < 8; ++a) wz[i * 8 + a] = ((sz + a) & 1) ? -w[a] : w[a];
   }
@@ -151,6 +153,31 @@ __global__ void k_prepare(NufftGeom g, uint64_t M, const float* __restrict__ kx,
   const int tx = sx / t.TX, ty = sy / t.TY, tz = sz / t.TZ;
   const int l = l0 ? l0[i] : 0;
   key[i] = (uint32_t)((((uint64_t)l * t.ntz + tz) * t.ntx + tx) * t.nty + ty);
+}
+
+// The order of the samples inside a subproblem: by window start (x, y, then z),
+// equal starts in binned order.  Neighbours in this order share windows, which
+// the spread sums in registers and the gather reads as one; along a stack's kz
+// they share all but two planes.  The 2-D gather's threads then read equal cells
+// too (128^2, L = 8, 4 coils: 41.2 -> 38.7 us per forward).  One block per subproblem, ranks by counting
+// (at most 512 samples).
+__global__ void k_order(const int4* __restrict__ sub, const uint32_t* __restrict__ perm,
+                        const uint2* __restrict__ start, uint32_t* __restrict__ order) {
+  __shared__ unsigned long long key[512];
+  const int4 sp = sub[blockIdx.x];
+  const int n = min(sp.w, 512);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const uint2 st = start[perm[sp.z + i]];
+    key[i] = (unsigned long long)(st.x & 0xffffu) << 48 | (unsigned long long)(st.x >> 16) << 32 |
+             (unsigned long long)(st.y & 0xffffu) << 16 | (unsigned long long)i;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const unsigned long long k = key[i];
+    int r = 0;
+    for (int j = 0; j < n; ++j) r += key[j] < k ? 1 : 0;
+    order[sp.z + r] = perm[sp.z + i];
+  }
 }
 
 __global__ void k_permute(uint64_t M, int dim, int K, const uint32_t* __restrict__ perm,
@@ -916,6 +943,156 @@ __global__ void __launch_bounds__(256, spread2d_min_blocks(CC * KK))
 }
 
 // ---------------------------------------------------------------------------
+// 3-D adjoint spread, segment windows of KK <= 3, CC coils per item.  Persistent
+// like k_spread2d.  The 8 warps of a block share the item's tile of float cells
+// without atomics: a window's 8 z taps fall one into each residue class mod 8,
+// so warp w takes of every sample the one tap with z = w (mod 8), and no two
+// warps ever touch one cell.  A warp's lane holds (y tap, x-tap pair) cells of the
+// current (x, y, z) in registers; it reads and writes the tile only when they
+// change.  Samples are ordered by window (k_order): along a stack's kz the next
+// window starts two cells on, and six of the eight warps keep their registers.
+// Cells are summed by one warp in sample order: deterministic, and in plain
+// FP32 (no fixed-point scale).
+// What bounds it is latency and issue at three blocks per SM (57 % of the issue
+// slots); the form before this one (one warp per sample, two int32 shared atomics
+// per cell, 32 per sample and plane) waited for the atomics.  Operator pairs on
+// one B200: 96^2 x 16, 8 coils, L = 6 1.86 -> 1.61 ms; 128^2 x 64, 2 shots, 4 coils,
+// L = 12 4.36 -> 4.12 ms.  The adjoint's error against 64 bits went from 1.4e-6 (the
+// fixed-point scale of a whole item) to 2e-7.
+// Tile layout [plane][15][15][16] float2, rows of odd x rotated by 8 cells: a
+// half-warp's two rows of 8 y taps fall into distinct banks.
+// ---------------------------------------------------------------------------
+namespace s3 {
+constexpr int T = 8, E = T + 7;           // tile edge, padded extent
+constexpr int CELLS = E * E * 16;         // cells of a plane
+constexpr int RUN = 64;                   // samples staged at a time
+__host__ __device__ constexpr size_t smem(int np) {
+  return (size_t)np * CELLS * sizeof(float2) + (size_t)RUN * (24 * sizeof(float) + np * sizeof(float2) + sizeof(int));
+}
+__device__ __forceinline__ int cell(int z, int x, int y) { return (z * E + x) * 16 + ((y + 8 * (x & 1)) & 15); }
+}  // namespace s3
+
+template <int CC, int KK>
+__global__ void __launch_bounds__(256) k_spread3d(NufftGeom g, TileShape t, const int4* __restrict__ sub,
+                                                  const uint2* __restrict__ start, const float* __restrict__ wxy,
+                                                  const float* __restrict__ wz, const uint32_t* __restrict__ perm,
+                                                  const float2* __restrict__ aa, const float2* __restrict__ y,
+                                                  uint64_t dstride, int nb, int L, float2* __restrict__ grids,
+                                                  unsigned* __restrict__ queue, int nchunks, int nitems) {
+  pdl_wait();
+  using namespace s3;
+  constexpr int NP = CC * KK;
+  extern __shared__ __align__(16) float2 sm3[];
+  float2* tile = sm3;
+  float* sw = reinterpret_cast<float*>(tile + NP * CELLS);          // [RUN][24]: wx, wy, wz
+  float2* sv = reinterpret_cast<float2*>(sw + RUN * 24);            // [RUN][NP]
+  int* sst = reinterpret_cast<int*>(sv + RUN * NP);                 // [RUN] window start in the tile
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int dy = lane & 7, dx = lane >> 3;
+  for (int q = tid; q < NP * CELLS / 2; q += 256) reinterpret_cast<float4*>(tile)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int item; (item = next_item(queue, nitems)) >= 0;) {
+    const int4 sp = sub[item / nchunks];
+    const int cfirst = (item % nchunks) * CC;
+    const int ncl = min(CC, nb - cfirst);
+    const int lseg = sp.y, first = sp.z, count = sp.w;
+    const int ty = sp.x % t.nty, txz = sp.x / t.nty, tx = txz % t.ntx, tz = txz / t.ntx;
+    const int x0 = tx * T, y0 = ty * T, z0 = tz * T;
+    float2 a0[NP], a1[NP];                 // cells (x + dx, y + dy) and (x + dx + 4, y + dy) at this warp's z
+#pragma unroll
+    for (int p = 0; p < NP; ++p) a0[p] = a1[p] = make_float2(0.f, 0.f);
+    int cur = -1;                          // ox | oy << 8 | z << 16 of the cells in registers
+    float2* c0 = tile;
+    auto put = [&]() {
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        float2* q = c0 + p * CELLS;
+        const float2 u = q[0], v = q[64];  // x + 4: 4 rows of 16
+        q[0] = make_float2(u.x + a0[p].x, u.y + a0[p].y);
+        q[64] = make_float2(v.x + a1[p].x, v.y + a1[p].y);
+        a0[p] = a1[p] = make_float2(0.f, 0.f);
+      }
+    };
+    for (int r0 = 0; r0 < count; r0 += RUN) {
+      const int n = min(RUN, count - r0);
+      if (r0) __syncthreads();             // the staged samples are no longer in use
+      for (int q = tid; q < n * 6; q += 256) {
+        const int i = q / 6, a = q - i * 6;
+        const uint64_t s = (uint64_t)(first + r0 + i);
+        const float4* src = a < 4 ? reinterpret_cast<const float4*>(wxy + s * 16) + a
+                                  : reinterpret_cast<const float4*>(wz + s * 8) + (a - 4);
+        cp_async16(reinterpret_cast<float4*>(sw + i * 24) + a, src);
+      }
+      for (int q = tid; q < n * CC; q += 256) {
+        const int i = q / CC, c = q - i * CC;
+        const uint64_t s = (uint64_t)(first + r0 + i);
+        float2 d = make_float2(0.f, 0.f);
+        if (c < ncl) {
+          const uint32_t ps = perm[s];
+          if (PG_CHECK(ps < dstride, PG_SITE_SPREAD2D_PERM, ps)) d = y[(uint64_t)(cfirst + c) * dstride + ps];
+        }
+#pragma unroll
+        for (int j = 0; j < KK; ++j) sv[i * NP + c * KK + j] = aa ? cmul(cconj(aa[s * KK + j]), d) : d;
+      }
+      if (tid < n) {
+        const uint2 st = start[first + r0 + tid];
+        const int ox = (int)(st.x & 0xffff) - x0, oy = (int)(st.x >> 16) - y0, oz = (int)st.y - z0;
+        sst[tid] = PG_CHECK(ox >= 0 && ox < T && oy >= 0 && oy < T && oz >= 0 && oz < T, PG_SITE_SPREAD_WINDOW,
+                            ox * 65536 + oy)
+                       ? ox | oy << 8 | oz << 16
+                       : -1;
+      }
+      cp_async_wait_all();
+      __syncthreads();
+      for (int i = 0; i < n; ++i) {
+        const int st = sst[i];
+        if (st < 0) continue;
+        const int oz = st >> 16;
+        const int e = (warp - oz) & 7;     // this warp's z tap
+        const float wzv = sw[i * 24 + 16 + e];
+        if (wzv == 0.f) continue;          // uniform across the warp
+        const int key = (st & 0xffff) | (oz + e) << 16;
+        if (key != cur) {
+          if (cur >= 0) put();
+          cur = key;
+          c0 = tile + cell(oz + e, (st & 0xff) + dx, (st >> 8 & 0xff) + dy);
+        }
+        const float wyz = sw[i * 24 + 8 + dy] * wzv;
+        const float w0 = sw[i * 24 + dx] * wyz, w1 = sw[i * 24 + dx + 4] * wyz;
+        const float2 w0v = make_float2(w0, w0), w1v = make_float2(w1, w1);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          const float2 v = sv[i * NP + p];
+          a0[p] = __ffma2_rn(w0v, v, a0[p]);
+          a1[p] = __ffma2_rn(w1v, v, a1[p]);
+        }
+      }
+    }
+    if (cur >= 0) put();
+    __syncthreads();
+    // flush two cells (y, y + 1) per vector atomic, zeroing them for the next item
+    const uint64_t G = g.ngrid();
+    for (int q = tid; q < E * E * 8; q += 256) {
+      const int row = q >> 3, yy = (q & 7) * 2;
+      const int zz = row / E, xx = row - zz * E;
+      float4* p4 = reinterpret_cast<float4*>(tile + cell(zz, xx, yy));
+      const int gx = x0 + xx, gy = y0 + yy, gz = z0 + zz;
+      const bool inside = gx < g.Gx && gy < g.Gy && gz < g.Gz;
+      const uint64_t idx = (uint64_t)gy + (uint64_t)g.Gy * ((uint64_t)gx + (uint64_t)g.Gx * gz);
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const int c = p / KK, j = p % KK;
+        const float4 v = p4[p * (CELLS / 2)];
+        if (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f) {
+          p4[p * (CELLS / 2)] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (inside && c < ncl)
+            atomicAdd(reinterpret_cast<float4*>(grids + ((uint64_t)(cfirst + c) * L + lseg + j) * G + idx), v);
+        }
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Adjoint post-kernel: crop the centred grid, undo the checkerboard,
 // deapodize, apply WoH, combine segments and coils.  CP x LP lanes share one
 // pixel: lane (c, h) takes coils c, c+CP, ... and segments h, h+LP, ...; the
@@ -1135,6 +1312,7 @@ std::unique_ptr<Binning> binning_share(const Binning& b) {
   o->K = b.K; o->L = b.L; o->M = b.M; o->tile = b.tile;
   o->nsub = b.nsub; o->submax = b.submax; o->nkeys = b.nkeys;
   o->perm.borrow(b.perm);
+  o->order.borrow(b.order);
   o->keys.borrow(b.keys);
   o->start.borrow(b.start);
   o->wxy.borrow(b.wxy);
@@ -1193,7 +1371,7 @@ pg_status nufft_build_binning(NufftPlan* p, int L, int K, const int* l0_host, co
   PG_CUDA(cudaStreamSynchronize(s));
 
   // Subproblems: each (segment window, tile) bin split into chunks.
-  const int kMaxPerSub = (g.dim == 2) ? p->tune.submax2d : p->tune.submax3d;
+  const int kMaxPerSub = std::min(512, (g.dim == 2) ? p->tune.submax2d : p->tune.submax3d);   // k_order's limit
   std::vector<int4> subs;
   for (uint64_t k = 0; k < b->nkeys; ++k) {
     const uint64_t a = starts[k], e = (k + 1 < b->nkeys) ? starts[k + 1] : M;
@@ -1219,7 +1397,9 @@ pg_status nufft_build_binning(NufftPlan* p, int L, int K, const int* l0_host, co
     PG_TRY(b->l0.alloc(M));
     PG_TRY(b->aa.alloc(M * (uint64_t)K));
   }
-  PG_LAUNCH(k_permute, ceil_div(M, 256), 256, 0, s, M, g.dim, K, b->perm.p, st_o.p, wxy_o.p,
+  PG_TRY(b->order.alloc(M));
+  PG_LAUNCH(k_order, (unsigned)b->nsub, 256, 0, s, b->subprob.p, b->perm.p, st_o.p, b->order.p);
+  PG_LAUNCH(k_permute, ceil_div(M, 256), 256, 0, s, M, g.dim, K, b->order.p, st_o.p, wxy_o.p,
             g.dim == 3 ? wz_o.p : nullptr, b->start.p, b->wxy.p, g.dim == 3 ? b->wz.p : nullptr,
             l0_host ? l0d.p : nullptr, l0_host ? aa_d.p : nullptr, l0_host ? b->l0.p : nullptr,
             l0_host ? b->aa.p : nullptr);
@@ -1429,7 +1609,7 @@ static pg_status gather_launch_one(NufftPlan* p, const Binning* bin, const float
   // a static grid: the persistent work-queue form measured ~4 % slower here
   dim3 grid(bin->nsub * (DIM == 2 ? 2 : 1), ceil_div(nb, CC));
   PG_LAUNCH_PDL((k_gather<DIM, T, CC, KP>), grid, 128, smem, s, p->g, bin->tile, bin->subprob.p, bin->start.p,
-            bin->wxy.p, bin->wz.p, bin->perm.p, aa, bin->K, bin->L, p->work->grids.p, nb, y, dstride);
+            bin->wxy.p, bin->wz.p, bin->order.p, aa, bin->K, bin->L, p->work->grids.p, nb, y, dstride);
   return PG_OK;
 }
 
@@ -1506,7 +1686,6 @@ static pg_status spread_launch_t(NufftPlan* p, const Binning* bin, const SpreadA
 
 static pg_status launch_spread(NufftPlan* p, const Binning* bin, const SpreadArgs& a, float2* target,
                                cudaStream_t s) {
-  if (p->g.dim == 3) return spread_launch_t<3, 8>(p, bin, a, target, s);
   if (bin->tile.TX == 32) return spread_launch_t<2, 32>(p, bin, a, target, s);
   return spread_launch_t<2, 16>(p, bin, a, target, s);
 }
@@ -1528,7 +1707,7 @@ static pg_status spread2d_launch(NufftPlan* p, const Binning* bin, const float2*
   PG_TRY(ensure_queue(p, s));
   const int blocks = persistent_blocks((const void*)k_spread2d<T, CC, KK>, smem, nitems);
   PG_LAUNCH_PDL((k_spread2d<T, CC, KK>), blocks, 256, smem, s, p->g, bin->tile, bin->subprob.p, bin->start.p, bin->wxy.p,
-            bin->perm.p, aa, y, dstride, nb, bin->L, bin->submax, wmax, target, p->work->queue.p, nchunks, nitems);
+            bin->order.p, aa, y, dstride, nb, bin->L, bin->submax, wmax, target, p->work->queue.p, nchunks, nitems);
   return PG_OK;
 }
 
@@ -1544,6 +1723,33 @@ static pg_status spread2d_launch_t(NufftPlan* p, const Binning* bin, int cc, con
     case 42: return spread2d_launch<T, 4, 2>(p, bin, aa, y, dstride, nb, wmax, target, s);
   }
   return set_error(PG_INVALID_ARG, "adjoint: no folded spread for %d coils x K=%d", cc, bin->K);
+}
+
+// 3-D: two planes per item (58 KB of tile: three blocks per SM), the K of one
+// coil, or two coils without segments.
+template <int CC, int KK>
+static pg_status spread3d_launch(NufftPlan* p, const Binning* bin, const float2* aa, const float2* y,
+                                 uint64_t dstride, int nb, float2* target, cudaStream_t s) {
+  const size_t smem = s3::smem(CC * KK);
+  PG_TRY(allow_full_dynamic_smem((const void*)k_spread3d<CC, KK>));
+  const int nchunks = (nb + CC - 1) / CC;
+  const int nitems = bin->nsub * nchunks;
+  PG_TRY(ensure_queue(p, s));
+  const int blocks = persistent_blocks((const void*)k_spread3d<CC, KK>, smem, nitems);
+  PG_LAUNCH_PDL((k_spread3d<CC, KK>), blocks, 256, smem, s, p->g, bin->tile, bin->subprob.p, bin->start.p, bin->wxy.p,
+                bin->wz.p, bin->order.p, aa, y, dstride, nb, bin->L, target, p->work->queue.p, nchunks, nitems);
+  return PG_OK;
+}
+
+static pg_status launch_spread3d(NufftPlan* p, const Binning* bin, const float2* aa, const float2* y,
+                                 uint64_t dstride, int nb, float2* target, cudaStream_t s) {
+  switch (bin->K) {
+    case 1: return nb > 1 ? spread3d_launch<2, 1>(p, bin, aa, y, dstride, nb, target, s)
+                          : spread3d_launch<1, 1>(p, bin, aa, y, dstride, nb, target, s);
+    case 2: return spread3d_launch<1, 2>(p, bin, aa, y, dstride, nb, target, s);
+    case 3: return spread3d_launch<1, 3>(p, bin, aa, y, dstride, nb, target, s);
+  }
+  return set_error(PG_INVALID_ARG, "adjoint: segment window K=%d too wide for shared memory", bin->K);
 }
 
 // Post-kernel launch: CP coil lanes x LP segment lanes per pixel (powers of
@@ -1643,11 +1849,13 @@ pg_status nufft_adjoint(NufftPlan* p, const NufftBatch& b, const float2* y, floa
     return plane_bytes * K * cc + (size_t)smax * (spread_wrow(g.dim) * sizeof(float) + sizeof(uint2) +
                                                   (size_t)K * cc * sizeof(float2));
   };
-  // 2-D with K <= 2 (Hanning segments or none): the folded spread reads the
+  // 3-D, and 2-D with K <= 2 (Hanning segments or none): the spread reads the
   // data vector itself; otherwise k_adjoint_prep forms the values first.
-  const bool folded = (g.dim == 2 && K <= 2 && (t.TX == 16 || t.TX == 32));
+  const bool folded = g.dim == 3 || (K <= 2 && (t.TX == 16 || t.TX == 32));
   int Cc = std::max(1, std::min(4, p->tune.spread_cc));
-  if (folded) {
+  if (g.dim == 3) {
+    if (K > 3) return set_error(PG_INVALID_ARG, "adjoint: segment window K=%d too wide for shared memory", K);
+  } else if (folded) {
     Cc = Cc >= 4 ? 4 : Cc >= 2 ? 2 : 1;
     while (Cc > 1 && (Cc >= 2 * std::min(Cb, b.C) || spread2d_smem(t.TX, Cc * K, smax) > smem_limit)) Cc >>= 1;
     if (spread2d_smem(t.TX, K, smax) > smem_limit)
@@ -1681,26 +1889,27 @@ pg_status nufft_adjoint(NufftPlan* p, const NufftBatch& b, const float2* y, floa
     ProfScope pag("adjoint_gridding", s);
     if (folded) {
       if (!self_clear) {
+        // the own 3-D passes read only the supported cells
         ProfScope ps("prep", s);
-        PG_CUDA(cudaMemsetAsync(target, 0, (size_t)B * G * sizeof(float2), s));
+        if (p->own_fft) PG_TRY(fftpass_clear(g, FftBatch{nb, L}, bin->sup, target, s));
+        else PG_CUDA(cudaMemsetAsync(target, 0, (size_t)B * G * sizeof(float2), s));
       }
       p->work->agrids_clean = false;
       if (bin->nsub > 0) {
         ProfScope ps("spread", s);
-        if (t.TX == 32) PG_TRY(spread2d_launch_t<32>(p, bin, Cc, aa, yc, b.data_stride, nb, wmax, target, s));
+        if (g.dim == 3) PG_TRY(launch_spread3d(p, bin, aa, yc, b.data_stride, nb, target, s));
+        else if (t.TX == 32) PG_TRY(spread2d_launch_t<32>(p, bin, Cc, aa, yc, b.data_stride, nb, wmax, target, s));
         else PG_TRY(spread2d_launch_t<16>(p, bin, Cc, aa, yc, b.data_stride, nb, wmax, target, s));
       }
     } else {
     PG_TRY(grow(p->work->vs, (uint64_t)nb * bin->M * K, s));
     {
       ProfScope ps("prep", s);
-      // a self-clearing target is already zero, and the own 3-D passes read
-      // only the supported cells: only cuFFT needs every cell cleared
-      if (p->own_fft && !self_clear) PG_TRY(fftpass_clear(g, FftBatch{nb, L}, bin->sup, target, s));
-      const uint64_t n4 = p->own_fft ? 0 : (uint64_t)B * G / 2;   // G is even: float2 pairs -> float4 words
+      // a self-clearing target is already zero: only the values are formed
+      const uint64_t n4 = self_clear ? 0 : (uint64_t)B * G / 2;   // G is even: float2 pairs -> float4 words
       const uint64_t work = std::max<uint64_t>(n4, bin->M);
       PG_LAUNCH(k_adjoint_prep, (unsigned)std::min<uint64_t>(ceil_div(work, 256), 8ull * sm_count()), 256, 0, s, n4,
-                reinterpret_cast<float4*>(target), nb, bin->M, K, bin->perm.p, aa, yc, b.data_stride,
+                reinterpret_cast<float4*>(target), nb, bin->M, K, bin->order.p, aa, yc, b.data_stride,
                 p->work->vs.p);
     }
     p->work->agrids_clean = false;

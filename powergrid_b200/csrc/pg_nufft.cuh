@@ -62,7 +62,9 @@ struct Binning {
   int L = 1;                 // segments
   uint64_t M = 0;            // samples
   TileShape tile{};
-  DevBuf<uint32_t> perm;     // sorted -> original sample index
+  DevBuf<uint32_t> perm;     // stable counting sort by bin: sorted -> original sample index
+  DevBuf<uint32_t> order;    // the same bins, ordered by window inside each subproblem; the
+                             // order of start, wxy, wz, l0 and aa
   DevBuf<uint2> start;       // (sx | sy << 16, sz): first of 8 taps per axis
   DevBuf<float> wxy;         // 16 per sample: wx[8], wy[8]
   DevBuf<float> wz;          // 8 per sample (3-D)
