@@ -316,47 +316,43 @@ __device__ __forceinline__ int next_item(unsigned* q, int nitems) {
 }
 
 // ---------------------------------------------------------------------------
-// Forward interpolation, tiled: one block per (subproblem, coil chunk), in 2-D
-// two for subproblems of more than kGatherHalf samples.  The
-// padded tiles of the subproblem's KP segment grids for CC coils are staged in
-// shared memory as complex cells ([c][j][PZ][PX][PY]).  Then one thread per
-// sample reads its 8^d cells of every (coil, segment) plane and sums them in
+// 2-D forward interpolation, tiled: one block per (subproblem, coil
+// chunk), two for subproblems of more than kGatherHalf samples.  The padded
+// tiles of the subproblem's KP segment grids for CC coils are staged in
+// shared memory as complex cells ([c][j][PX][PY]).  Then one thread per
+// sample reads its 64 cells of every (coil, segment) plane and sums them in
 // the reference's order (x outer, y inner, gridding.cpp:275-289) with paired
 // fma; no cross-lane reduction is needed, and consecutive samples of a warp
 // often share their window (spiral readouts are oversampled along the arm),
 // so their shared-memory reads broadcast.  The segment interpolator AA is
 // applied per coil on the way out.
 // ---------------------------------------------------------------------------
-constexpr int kGatherHalf = 128;   // 2-D subproblems above this are gathered by two blocks
+constexpr int kGatherHalf = 128;   // subproblems above this are gathered by two blocks
 
-template <int DIM, int T, int CC, int KP>
+template <int T, int CC, int KP>
 __global__ void __launch_bounds__(128) k_gather(NufftGeom g, TileShape t, const int4* __restrict__ sub,
-                                                const uint2* __restrict__ start, const float* __restrict__ wxy,
-                                                const float* __restrict__ wz, const uint32_t* __restrict__ perm,
+                                                const uint2* __restrict__ start,
+                                                const float* __restrict__ wxy, const uint32_t* __restrict__ perm,
                                                 const float2* __restrict__ aa, int K, int L,
                                                 const float2* __restrict__ grids, int Cb,
                                                 float2* __restrict__ data, uint64_t dstride) {
   pdl_wait();
-  using TG = TileGeo<DIM, T>;
-  constexpr int CELLS = TG::CELLS, PY = TG::PY, PX = TG::PX, PLANE = TG::PLANE;
-  extern __shared__ __align__(16) float2 sm2[];   // [c*KP + j][PZ][PX][PY] complex cells
-  // In 2-D two blocks share a subproblem of more than kGatherHalf samples,
+  using TG = TileGeo<2, T>;
+  constexpr int CELLS = TG::CELLS, PY = TG::PY;
+  extern __shared__ __align__(16) float2 sm2[];   // [c*KP + j][PX][PY] complex cells
+  // Two blocks share a subproblem of more than kGatherHalf samples,
   // one per half (more blocks to cover the staging latency; each stages the
   // tile); the second block of a smaller subproblem has nothing to do.
-  constexpr int SPLIT = (DIM == 2) ? 2 : 1;
+  constexpr int SPLIT = 2;
   const int4 sp = sub[blockIdx.x / SPLIT];
   const int part = blockIdx.x % SPLIT;
-  const int head = (SPLIT == 2 && sp.w > kGatherHalf) ? (sp.w + 1) / 2 : sp.w;
+  const int head = (sp.w > kGatherHalf) ? (sp.w + 1) / 2 : sp.w;
   const int first = sp.z + part * head, count = part ? sp.w - head : head;
   if (count <= 0) return;
   const int cfirst = blockIdx.y * CC;
   const int ncl = min(CC, Cb - cfirst);
   const int tile = sp.x, lseg = sp.y;
-  const int ty = tile % t.nty;
-  const int txz = tile / t.nty;
-  const int tx = txz % t.ntx;
-  const int tz = txz / t.ntx;
-  const int x0 = tx * T, y0 = ty * T, z0 = tz * TG::TZ;
+  const int x0 = (tile / t.nty) * T, y0 = (tile % t.nty) * T;
   const uint64_t G = g.ngrid();
   // cell pairs (y, y+1) with asynchronous 16-byte copies: PY, y0 and Gy are
   // even, so a pair is in the grid or outside it as a whole and both of its
@@ -364,12 +360,9 @@ __global__ void __launch_bounds__(128) k_gather(NufftGeom g, TileShape t, const 
   static_assert(PY % 2 == 0 && CELLS % 2 == 0, "cell pairs");
   for (int t2 = threadIdx.x; t2 < CELLS / 2; t2 += blockDim.x) {
     const int q = 2 * t2;
-    const int pyy = q % PY;
-    const int pxx = (q / PY) % PX;
-    const int pzz = q / PLANE;
-    const int gy = y0 + pyy, gx = x0 + pxx, gz = z0 + pzz;
-    const bool in = gy < g.Gy && gx < g.Gx && gz < g.Gz;
-    const uint64_t idx = (uint64_t)gy + (uint64_t)g.Gy * ((uint64_t)gx + (uint64_t)g.Gx * gz);
+    const int gy = y0 + q % PY, gx = x0 + q / PY;
+    const bool in = gy < g.Gy && gx < g.Gx;
+    const uint64_t idx = (uint64_t)gy + (uint64_t)g.Gy * (uint64_t)gx;
 #pragma unroll
     for (int c = 0; c < CC; ++c)
 #pragma unroll
@@ -387,10 +380,7 @@ __global__ void __launch_bounds__(128) k_gather(NufftGeom g, TileShape t, const 
   for (int s = first + threadIdx.x; s < end; s += blockDim.x) {
     const uint2 st = start[s];
     const int ox = (int)(st.x & 0xffff) - x0, oy = (int)(st.x >> 16) - y0;
-    if (!PG_CHECK(ox >= 0 && ox < T && oy >= 0 && oy < T &&
-                      (DIM == 2 || ((int)st.y - z0 >= 0 && (int)st.y - z0 < TG::TZ)),
-                  PG_SITE_GATHER_WINDOW, ox * 65536 + oy))
-      continue;
+    if (!PG_CHECK(ox >= 0 && ox < T && oy >= 0 && oy < T, PG_SITE_GATHER_WINDOW, ox * 65536 + oy)) continue;
     const float4* w4 = reinterpret_cast<const float4*>(wxy + (uint64_t)s * 16);
     const float4 wa = w4[0], wb = w4[1], wc = w4[2], wd = w4[3];
     const float wxr[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
@@ -399,34 +389,15 @@ __global__ void __launch_bounds__(128) k_gather(NufftGeom g, TileShape t, const 
 #pragma unroll
     for (int i = 0; i < CC * KP; ++i) acc[i] = make_float2(0.f, 0.f);
     const float2* base = sm2 + ox * PY + oy;
-    if (DIM == 2) {
 #pragma unroll
-      for (int r = 0; r < 8; ++r)
+    for (int r = 0; r < 8; ++r)
 #pragma unroll
-        for (int d = 0; d < 8; ++d) {
-          const float w = wxr[r] * wyr[d];
-          const float2 w2 = make_float2(w, w);
+      for (int d = 0; d < 8; ++d) {
+        const float w = wxr[r] * wyr[d];
+        const float2 w2 = make_float2(w, w);
 #pragma unroll
-          for (int cj = 0; cj < CC * KP; ++cj) acc[cj] = __ffma2_rn(w2, base[cj * CELLS + r * PY + d], acc[cj]);
-        }
-    } else {
-      const int oz = (int)st.y - z0;
-      const float* wzz = wz + (uint64_t)s * 8;
-      const float2* bz = base + oz * PLANE;
-#pragma unroll 1
-      for (int e = 0; e < 8; ++e, bz += PLANE) {
-        const float wze = wzz[e];
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-          for (int d = 0; d < 8; ++d) {
-            const float w = wxr[r] * wyr[d] * wze;
-            const float2 w2 = make_float2(w, w);
-#pragma unroll
-            for (int cj = 0; cj < CC * KP; ++cj) acc[cj] = __ffma2_rn(w2, bz[cj * CELLS + r * PY + d], acc[cj]);
-          }
+        for (int cj = 0; cj < CC * KP; ++cj) acc[cj] = __ffma2_rn(w2, base[cj * CELLS + r * PY + d], acc[cj]);
       }
-    }
     const uint32_t o = perm[s];
     if (!PG_CHECK(o < dstride, PG_SITE_GATHER_PERM, o)) continue;
 #pragma unroll
@@ -440,6 +411,125 @@ __global__ void __launch_bounds__(128) k_gather(NufftGeom g, TileShape t, const 
           if (j < K) out = cadd(out, cmul(acc[c * KP + j], aa[(uint64_t)s * K + j]));
       }
       data[(uint64_t)(cfirst + c) * dstride + o] = out;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// 3-D forward interpolation: eight lanes per sample, lane = y tap, straight from
+// the grid.  A lane walks its window's x and z taps and sums CC coils x KP
+// segments of them in registers with paired fma; the segment interpolator AA is
+// applied per lane, and the coils' sums over the eight lanes are formed by
+// halving exchanges (each step halves the coils a lane keeps).  A group's load is
+// one 64-byte row of the window; consecutive samples are neighbours (binned
+// order, readouts oversampled along the arm), so a block's windows overlap and
+// are served by L1, and equal windows in a warp by one access.
+// What bounds it is L1: 512 cells of 8 bytes per sample and plane (80 % busy).
+// It replaces tiles staged in shared memory: a bin holds some 30 samples of a
+// segment, its padded tile 6144 cells per plane (98 KB, two blocks per SM).
+// Operator pairs on one B200: 96^2 x 16, 8 coils, L = 6 1.61 -> 1.10 ms; 128^2 x 64,
+// 2 shots, 4 coils, L = 12 4.12 -> 3.35 ms.  In 2-D the staged tiles of k_gather stay:
+// 38.7 against 46.6 us at 128^2 (2 samples per cell), 345 against 346 us at 208^2
+// (0.6 per cell).
+// Taps outside the clamped window weigh 0 and, where they lie outside the grid,
+// are not read.
+// ---------------------------------------------------------------------------
+constexpr int kGatherRun = 64;    // samples per block: two passes of 32
+
+template <int CC, int KP>
+__global__ void __launch_bounds__(256) k_gather3d(NufftGeom g, uint64_t M, const uint2* __restrict__ start,
+                                                  const float* __restrict__ wxy, const float* __restrict__ wz,
+                                                  const uint32_t* __restrict__ perm, const int* __restrict__ l0,
+                                                  const float2* __restrict__ aa, int K, int L,
+                                                  const float2* __restrict__ grids, int Cb,
+                                                  float2* __restrict__ data, uint64_t dstride) {
+  pdl_wait();
+  const int cfirst = blockIdx.y * CC;
+  const int ncl = min(CC, Cb - cfirst);
+  const uint64_t G = g.ngrid();
+  const int a = threadIdx.x & 7;                      // y tap
+#pragma unroll 1
+  for (int pass = 0; pass < kGatherRun / 32; ++pass) {
+    const uint64_t s0 = (uint64_t)blockIdx.x * kGatherRun + pass * 32 + (threadIdx.x >> 3);
+    if (s0 - (threadIdx.x >> 3 & 3) >= M) continue;   // the whole warp is past the end
+    const uint64_t s = s0 < M ? s0 : M - 1;
+    const uint2 st = start[s];
+    const int sx = (int)(st.x & 0xffff), sy = (int)(st.x >> 16), sz = (int)st.y;
+    const int ls = l0 ? l0[s] : 0;
+    const float4* w4 = reinterpret_cast<const float4*>(wxy + s * 16);
+    const float4 wa = w4[0], wb = w4[1];
+    const float wx[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+    const float wy = wxy[s * 16 + 8 + a];
+    // taps inside the grid along x and z; lanes past its y edge read nothing
+    const int nx = min(8, g.Gx - sx), nz = min(8, g.Gz - sz);
+    const bool in = sy + a < g.Gy && nx > 0 && nz > 0 && PG_CHECK(ls >= 0 && ls + K <= L, PG_SITE_GATHER_WINDOW, ls);
+    float2 acc[CC * KP];
+#pragma unroll
+    for (int i = 0; i < CC * KP; ++i) acc[i] = make_float2(0.f, 0.f);
+    if (in) {
+      const float2* p = grids + ((uint64_t)cfirst * L + ls) * G + (uint64_t)(sy + a) +
+                        (uint64_t)g.Gy * ((uint64_t)sx + (uint64_t)g.Gx * sz);
+      const uint64_t cstep = (uint64_t)L * G, zstep = (uint64_t)g.Gx * g.Gy;
+#pragma unroll 1
+      for (int z = 0; z < nz; ++z, p += zstep) {
+        const float wyz = wy * wz[s * 8 + z];
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+          const float w = wx[x] * wyz;
+          const float2 w2 = make_float2(w, w);
+          // past the edge the weight is 0: read the last row again
+          const float2* q = p + (uint64_t)((unsigned)min(x, nx - 1) * (unsigned)g.Gy);
+#pragma unroll
+          for (int c = 0; c < CC; ++c)
+#pragma unroll
+            for (int j = 0; j < KP; ++j)
+              if ((CC == 1 || c < ncl) && (KP <= 2 || j < K))
+                acc[c * KP + j] = __ffma2_rn(w2, q[(uint64_t)c * cstep + (uint64_t)j * G], acc[c * KP + j]);
+        }
+      }
+    }
+    // apply the interpolator, then sum over the eight lanes
+    float2 v[CC];
+#pragma unroll
+    for (int c = 0; c < CC; ++c) v[c] = acc[c * KP];
+    if (aa) {
+#pragma unroll
+      for (int j = 0; j < KP; ++j) {
+        if (KP > 2 && j >= K) break;
+        const float2 f = aa[s * K + j];
+#pragma unroll
+        for (int c = 0; c < CC; ++c) {
+          const float2 t = cmul(acc[c * KP + j], f);
+          v[c] = j == 0 ? t : cadd(v[c], t);
+        }
+      }
+    }
+    int coil = 0;                                     // the coil this lane ends up with
+    int left = CC;
+#pragma unroll
+    for (int o = 4; o >= 1; o >>= 1) {
+      if (left > 1) {
+        const int h = left / 2;
+        const bool up = (a & o) != 0;
+#pragma unroll
+        for (int c = 0; c < CC / 2; ++c)
+          if (c < h) {
+            const float2 keep = up ? v[c + h] : v[c], give = up ? v[c] : v[c + h];
+            v[c] = make_float2(keep.x + __shfl_xor_sync(0xffffffffu, give.x, o),
+                               keep.y + __shfl_xor_sync(0xffffffffu, give.y, o));
+          }
+        coil += up ? h : 0;
+        left = h;
+      } else {
+        v[0].x += __shfl_xor_sync(0xffffffffu, v[0].x, o);
+        v[0].y += __shfl_xor_sync(0xffffffffu, v[0].y, o);
+      }
+    }
+    // lanes that differ only in the bits below the last halving hold the same coil
+    constexpr int kSame = 8 / CC;
+    if (s0 < M && (a & (kSame - 1)) == 0 && coil < ncl) {
+      const uint32_t o = perm[s];
+      if (PG_CHECK(o < dstride, PG_SITE_GATHER_PERM, o)) data[(uint64_t)(cfirst + coil) * dstride + o] = v[0];
     }
   }
 }
@@ -1157,7 +1247,7 @@ NufftPlan::~NufftPlan() {
   for (auto& kv : ffts) fft_release_plan(g, kv.first, kv.second.first, kv.second.second);
 }
 
-NufftTune NufftTune::defaults() {
+NufftTune NufftTune::defaults(int dim) {
   NufftTune t;
   auto env = [](const char* n, int d) {
     const char* v = getenv(n);
@@ -1168,7 +1258,7 @@ NufftTune NufftTune::defaults() {
   t.submax2d = env("PG_SUBMAX2D", t.submax2d);
   t.submax3d = env("PG_SUBMAX3D", t.submax3d);
   t.spread_cc = env("PG_SPREAD_CC", t.spread_cc);
-  t.gather_cc = env("PG_GATHER_CC", t.gather_cc);
+  t.gather_cc = env("PG_GATHER_CC", dim == 3 ? 1 : t.gather_cc);
   return t;
 }
 
@@ -1208,7 +1298,7 @@ pg_status nufft_plan_create(std::unique_ptr<NufftPlan>* out, uint64_t M, float g
                        (unsigned long long)i);
   }
   auto p = std::make_unique<NufftPlan>();
-  p->tune = NufftTune::defaults();
+  p->tune = NufftTune::defaults(nz == 1 ? 2 : 3);
   NufftGeom& g = p->g;
   g.dim = (nz == 1) ? 2 : 3;
   g.Nx = nx; g.Ny = ny; g.Nz = nz;
@@ -1601,50 +1691,84 @@ static pg_status ensure_queue(NufftPlan* p, cudaStream_t s) {
 // Tiled gather launch: choose the padded segment count KP and the coils per
 // block CC so that the staged tiles fit in shared memory and the per-thread
 // accumulators (2*CC*KP floats) stay at most 32.
-template <int DIM, int T, int CC, int KP>
+template <int T, int CC, int KP>
 static pg_status gather_launch_one(NufftPlan* p, const Binning* bin, const float2* aa, int nb, float2* y,
                                    uint64_t dstride, cudaStream_t s) {
-  const size_t smem = (size_t)CC * KP * 2 * TileGeo<DIM, T>::CELLS * sizeof(float);
-  PG_CUDA(cudaFuncSetAttribute(k_gather<DIM, T, CC, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const size_t smem = (size_t)CC * KP * 2 * TileGeo<2, T>::CELLS * sizeof(float);
+  PG_CUDA(cudaFuncSetAttribute(k_gather<T, CC, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // a static grid: the persistent work-queue form measured ~4 % slower here
-  dim3 grid(bin->nsub * (DIM == 2 ? 2 : 1), ceil_div(nb, CC));
-  PG_LAUNCH_PDL((k_gather<DIM, T, CC, KP>), grid, 128, smem, s, p->g, bin->tile, bin->subprob.p, bin->start.p,
-            bin->wxy.p, bin->wz.p, bin->order.p, aa, bin->K, bin->L, p->work->grids.p, nb, y, dstride);
+  dim3 grid(bin->nsub * 2, ceil_div(nb, CC));
+  PG_LAUNCH_PDL((k_gather<T, CC, KP>), grid, 128, smem, s, p->g, bin->tile, bin->subprob.p, bin->start.p,
+            bin->wxy.p, bin->order.p, aa, bin->K, bin->L, p->work->grids.p, nb, y, dstride);
   return PG_OK;
 }
 
-template <int DIM, int T>
+template <int T>
 static pg_status launch_gather_t(NufftPlan* p, const Binning* bin, const float2* aa, int nb, float2* y,
                                  uint64_t dstride, cudaStream_t s) {
   const int K = bin->K;
   const int KP = K <= 1 ? 1 : K <= 2 ? 2 : K <= 4 ? 4 : 8;
-  const size_t pair = (size_t)TileGeo<DIM, T>::CELLS * 2 * sizeof(float);
+  const size_t pair = (size_t)TileGeo<2, T>::CELLS * 2 * sizeof(float);
   const size_t limit = (size_t)smem_optin_bytes() - 6144;  // static reduction buffer + margin
   int CC = std::max(1, std::min(4, p->tune.gather_cc));
   while (CC > 1 && (CC >= 2 * nb || 2 * CC * KP > 32 || (size_t)CC * KP * pair > limit)) CC >>= 1;
   if ((size_t)CC * KP * pair > limit || 2 * CC * KP > 32)
     return set_error(PG_INVALID_ARG, "forward: segment window K=%d too wide for shared memory", K);
   switch (KP * 10 + CC) {
-    case 11: return gather_launch_one<DIM, T, 1, 1>(p, bin, aa, nb, y, dstride, s);
-    case 12: return gather_launch_one<DIM, T, 2, 1>(p, bin, aa, nb, y, dstride, s);
-    case 14: return gather_launch_one<DIM, T, 4, 1>(p, bin, aa, nb, y, dstride, s);
-    case 21: return gather_launch_one<DIM, T, 1, 2>(p, bin, aa, nb, y, dstride, s);
-    case 22: return gather_launch_one<DIM, T, 2, 2>(p, bin, aa, nb, y, dstride, s);
-    case 24: return gather_launch_one<DIM, T, 4, 2>(p, bin, aa, nb, y, dstride, s);
-    case 41: return gather_launch_one<DIM, T, 1, 4>(p, bin, aa, nb, y, dstride, s);
-    case 42: return gather_launch_one<DIM, T, 2, 4>(p, bin, aa, nb, y, dstride, s);
-    case 44: return gather_launch_one<DIM, T, 4, 4>(p, bin, aa, nb, y, dstride, s);
-    case 81: return gather_launch_one<DIM, T, 1, 8>(p, bin, aa, nb, y, dstride, s);
-    case 82: return gather_launch_one<DIM, T, 2, 8>(p, bin, aa, nb, y, dstride, s);
+    case 11: return gather_launch_one<T, 1, 1>(p, bin, aa, nb, y, dstride, s);
+    case 12: return gather_launch_one<T, 2, 1>(p, bin, aa, nb, y, dstride, s);
+    case 14: return gather_launch_one<T, 4, 1>(p, bin, aa, nb, y, dstride, s);
+    case 21: return gather_launch_one<T, 1, 2>(p, bin, aa, nb, y, dstride, s);
+    case 22: return gather_launch_one<T, 2, 2>(p, bin, aa, nb, y, dstride, s);
+    case 24: return gather_launch_one<T, 4, 2>(p, bin, aa, nb, y, dstride, s);
+    case 41: return gather_launch_one<T, 1, 4>(p, bin, aa, nb, y, dstride, s);
+    case 42: return gather_launch_one<T, 2, 4>(p, bin, aa, nb, y, dstride, s);
+    case 44: return gather_launch_one<T, 4, 4>(p, bin, aa, nb, y, dstride, s);
+    case 81: return gather_launch_one<T, 1, 8>(p, bin, aa, nb, y, dstride, s);
+    case 82: return gather_launch_one<T, 2, 8>(p, bin, aa, nb, y, dstride, s);
+  }
+  return set_error(PG_INVALID_ARG, "forward: unsupported tiling (K=%d)", K);
+}
+
+// 3-D gather launch: CC coils x KP segments per pass, at most 8 planes (16
+// accumulator registers and 8 loads in flight per tap).  The tuner takes one
+// coil at the configurations' sizes: 48 registers, twice the warps of four coils.
+template <int CC, int KP>
+static pg_status gather3d_launch_one(NufftPlan* p, const Binning* bin, const float2* aa, int nb, float2* y,
+                                   uint64_t dstride, cudaStream_t s) {
+  const dim3 grid(ceil_div(bin->M, kGatherRun), ceil_div(nb, CC));
+  PG_LAUNCH_PDL((k_gather3d<CC, KP>), grid, 256, 0, s, p->g, bin->M, bin->start.p, bin->wxy.p, bin->wz.p,
+                bin->order.p, bin->l0.p, aa, bin->K, bin->L, p->work->grids.p, nb, y, dstride);
+  return PG_OK;
+}
+
+static pg_status launch_gather3d(NufftPlan* p, const Binning* bin, const float2* aa, int nb, float2* y,
+                               uint64_t dstride, cudaStream_t s) {
+  const int K = bin->K;
+  const int KP = K <= 1 ? 1 : K <= 2 ? 2 : 4;
+  if (K > 3) return set_error(PG_INVALID_ARG, "forward: segment window K=%d too wide", K);
+  int CC = 8 / KP;
+  while (CC > 1 && (CC >= 2 * nb || CC > p->tune.gather_cc)) CC >>= 1;
+  switch (KP * 10 + CC) {
+    case 11: return gather3d_launch_one<1, 1>(p, bin, aa, nb, y, dstride, s);
+    case 12: return gather3d_launch_one<2, 1>(p, bin, aa, nb, y, dstride, s);
+    case 14: return gather3d_launch_one<4, 1>(p, bin, aa, nb, y, dstride, s);
+    case 18: return gather3d_launch_one<8, 1>(p, bin, aa, nb, y, dstride, s);
+    case 21: return gather3d_launch_one<1, 2>(p, bin, aa, nb, y, dstride, s);
+    case 22: return gather3d_launch_one<2, 2>(p, bin, aa, nb, y, dstride, s);
+    case 24: return gather3d_launch_one<4, 2>(p, bin, aa, nb, y, dstride, s);
+    case 41: return gather3d_launch_one<1, 4>(p, bin, aa, nb, y, dstride, s);
+    case 42: return gather3d_launch_one<2, 4>(p, bin, aa, nb, y, dstride, s);
   }
   return set_error(PG_INVALID_ARG, "forward: unsupported tiling (K=%d)", K);
 }
 
 static pg_status launch_gather(NufftPlan* p, const Binning* bin, const float2* aa, int nb, float2* y,
                                uint64_t dstride, cudaStream_t s) {
-  if (p->g.dim == 3) return launch_gather_t<3, 8>(p, bin, aa, nb, y, dstride, s);
-  if (bin->tile.TX == 32) return launch_gather_t<2, 32>(p, bin, aa, nb, y, dstride, s);
-  return launch_gather_t<2, 16>(p, bin, aa, nb, y, dstride, s);
+  if (p->g.dim == 3) return launch_gather3d(p, bin, aa, nb, y, dstride, s);
+  if (bin->nsub == 0) return PG_OK;
+  if (bin->tile.TX == 32) return launch_gather_t<32>(p, bin, aa, nb, y, dstride, s);
+  return launch_gather_t<16>(p, bin, aa, nb, y, dstride, s);
 }
 
 // Spread launch arguments shared by every instantiation.
@@ -1828,7 +1952,7 @@ pg_status nufft_forward(NufftPlan* p, const NufftBatch& b, const float2* x, floa
     float2* yc = y + (uint64_t)c0 * b.data_stride;
     const float2* aa = (L > 1 || bin->aa.p) ? bin->aa.p : nullptr;
     ProfScope ps("gather", s);
-    if (bin->nsub > 0) PG_TRY(launch_gather(p, bin, aa, nb, yc, b.data_stride, s));
+    PG_TRY(launch_gather(p, bin, aa, nb, yc, b.data_stride, s));
   }
   return PG_OK;
 }

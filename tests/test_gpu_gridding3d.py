@@ -1,0 +1,69 @@
+"""3-D gridding at the edges of its tiles, items and windows, against the oracle.
+
+The spread's tiles have 8 cells per axis and its items at most 512 samples,
+staged 64 at a time; a window has 8 taps per axis, and samples of one window
+are summed before they reach the tile.  Tolerance: 1e-5 relative L2, the
+operator tolerance of the other parity tests (float windows and tables; the
+sums themselves are 32-bit)."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+OP_TOL = 1e-5
+
+
+def _trajectory(kind, n, nz):
+    r = np.random.default_rng(5)
+    if kind == "cluster":        # many samples per tile: several items, runs of equal windows
+        k = r.random((3, 3000)) * 1.5 - 0.75
+        k[:, ::7] = k[:, :1]
+    elif kind == "stack":        # one in-plane position over all kz, on and off the grid's planes
+        k = np.stack([np.full(4 * nz, 1.3), np.full(4 * nz, -2.6), np.linspace(-nz / 2, nz / 2 - 0.25, 4 * nz)])
+    elif kind == "tile_edges":   # window starts on both sides of every tile edge
+        c = (np.arange(2 * n) / 2.0 - n / 2)[:, None] + np.array([-0.01, 0.0, 0.01])
+        c = np.clip(c.ravel(), -n / 2, n / 2 - 0.01)
+        k = np.stack([c, r.permutation(c), r.random(c.size) * (nz - 0.1) - nz / 2])
+    else:                        # the border of k-space, and samples whose window is cut or lies past the grid
+        e = np.array([-1.0, -0.999, 0.98, 0.999, 1.0, 1.02, 1.04])
+        g = np.stack(np.meshgrid(e * n / 2, e * n / 2, e * nz / 2, indexing="ij")).reshape(3, -1)
+        k = g
+    return k.astype(np.float32)
+
+
+@pytest.mark.parametrize("n,nz,kind", [(16, 8, "cluster"), (16, 8, "stack"), (24, 9, "tile_edges"), (88, 8, "border"),
+                                       (16, 16, "border")])
+def test_gridding_3d_vs_oracle(pg, oracle, n, nz, kind):
+    from powergrid_b200 import synthetic as S
+    kx, ky, kz = _trajectory(kind, n, nz)
+    M, N = kx.size, n * n * nz
+    G, ref = pg.Gnufft(M, 2.0, n, n, nz, kx, ky, kz), oracle.gnufft(0, M, n, n, nz, kx, ky, kz)
+    x, y = S.image(S.Rng(3), N), S.image(S.Rng(4), M)
+    assert rel_l2(G * x, ref.forward(x)) <= OP_TOL
+    for _ in range(2):           # the second adjoint finds the grids as the first one left them
+        assert rel_l2(G / y, ref.adjoint(y)) <= OP_TOL
+
+
+@pytest.mark.parametrize("L,interp,nc", [(1, 1, 1), (1, 1, 2), (1, 1, 5), (4, 1, 1), (4, 1, 3), (3, 2, 2), (2, 1, 9)])
+def test_gridding_3d_planes_vs_oracle(pg, oracle, L, interp, nc):
+    """Every number of planes per item: window widths K = 1, 2, 3 and odd coil counts."""
+    from powergrid_b200 import synthetic as S
+    n, nz = 16, 8
+    kx, ky, kz, t = S.stack_of_spirals(n, nz, 2, 200, 8e-3)
+    M, N = kx.size, n * n * nz
+    fm, sm = S.field_map(S.Rng(1), n, n, nz, 60.0), S.coil_maps(S.Rng(2), n, n, nz, nc)
+    A, Ao = pg.Gnufft(M, 2.0, n, n, nz, kx, ky, kz), oracle.gnufft(0, M, n, n, nz, kx, ky, kz)
+    if L > 1:
+        A = pg.TimeSegmentation(A, fm, t, M, N, L, interp, 1)
+        Ao = oracle.timeseg(Ao, fm, t, M, N, L) if interp == 1 else None
+    x, y = S.image(S.Rng(3), N), S.image(S.Rng(4), M * nc)
+    Sg = pg.SENSE(A, sm, M, N, nc)
+    if Ao is None:               # dense windows: forward and adjoint are each other's transpose
+        a, b = np.vdot(Sg * x, y), np.vdot(x, Sg / y)
+        assert abs(a - b) <= OP_TOL * abs(a) + 1e-6 * np.linalg.norm(Sg * x) * np.linalg.norm(y)
+        return
+    So = oracle.sense(Ao, sm, M, N, nc)
+    assert rel_l2(Sg * x, So.forward(x)) <= OP_TOL
+    assert rel_l2(Sg / y, So.adjoint(y)) <= OP_TOL
