@@ -284,16 +284,13 @@ __host__ __device__ constexpr int padded_y(int T) {
   return py;
 }
 
-// Compile-time tile geometry: every shared-memory address in the gridding
+// Compile-time 2-D tile geometry: every shared-memory address in the gridding
 // loops is a per-sample base plus an immediate offset.
-template <int DIM, int T>
+template <int T>
 struct TileGeo {
-  static constexpr int TZ = (DIM == 3) ? T : 1;
   static constexpr int PX = T + 8;
   static constexpr int PY = padded_y(T);
-  static constexpr int PZ = (DIM == 3) ? T + 8 : 1;
-  static constexpr int PLANE = PX * PY;
-  static constexpr int CELLS = PLANE * PZ;
+  static constexpr int CELLS = PX * PY;
 };
 
 // Device work queue of the persistent spread launch: items are (subproblem,
@@ -337,7 +334,7 @@ __global__ void __launch_bounds__(128) k_gather(NufftGeom g, TileShape t, const 
                                                 const float2* __restrict__ grids, int Cb,
                                                 float2* __restrict__ data, uint64_t dstride) {
   pdl_wait();
-  using TG = TileGeo<2, T>;
+  using TG = TileGeo<T>;
   constexpr int CELLS = TG::CELLS, PY = TG::PY;
   extern __shared__ __align__(16) float2 sm2[];   // [c*KP + j][PX][PY] complex cells
   // Two blocks share a subproblem of more than kGatherHalf samples,
@@ -535,7 +532,7 @@ __global__ void __launch_bounds__(256) k_gather3d(NufftGeom g, uint64_t M, const
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint spread, persistent: as many blocks as fit on the device take
+// 2-D adjoint spread of segment windows K > 2, persistent: as many blocks as fit on the device take
 // (subproblem, coil chunk) items from a device work queue, largest first.
 //  1. The subproblem's samples are staged in shared memory with coalesced
 //     loads: tap starts, tap weights and, per (coil, segment) plane, the value
@@ -553,7 +550,7 @@ __global__ void __launch_bounds__(256) k_gather3d(NufftGeom g, uint64_t M, const
 //     not depend on the order of the atomics, so the result is deterministic.
 //  4. Each nonzero tile cell is flushed to the centred grid with one vector
 //     atomic, scaled back by 2^-e.
-// Tile layout [coil][segment][re|im][PZ][PX][PY], PY = 8 (mod 32): a warp's
+// Tile layout [coil][segment][re|im][PX][PY], PY = 8 (mod 32): a warp's
 // 32 lanes (8 y-taps x 4 x-taps) hit 32 distinct banks.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int fixed_point(float w, float v) {
@@ -561,20 +558,16 @@ __device__ __forceinline__ int fixed_point(float w, float v) {
   return __float_as_int(__fmaf_rn(w, v, kMagic)) - 0x4B400000;
 }
 
-// Staged weights per sample in the spread: wx[8], wy[8] and, in 3-D, wz[8].
-__host__ __device__ constexpr int spread_wrow(int dim) { return dim == 2 ? 16 : 24; }
-
-template <int DIM, int T, int NP>
+template <int T, int NP>
 __global__ void __launch_bounds__(256) k_spread(NufftGeom g, TileShape t, const int4* __restrict__ sub,
                                                 const uint2* __restrict__ start, const float* __restrict__ wxy,
-                                                const float* __restrict__ wz, const float2* __restrict__ vs,
-                                                uint64_t M, int K, int L, int c0, int cc, int smax, float wmax,
+                                                const float2* __restrict__ vs, uint64_t M, int K, int L, int c0, int cc, int smax, float wmax,
                                                 float2* __restrict__ grids, unsigned* __restrict__ queue,
                                                 int nchunks, int nitems) {
   pdl_wait();
-  using TG = TileGeo<DIM, T>;
-  constexpr int CELLS = TG::CELLS, PY = TG::PY, PX = TG::PX, PLANE = TG::PLANE;
-  constexpr int WROW = spread_wrow(DIM);   // staged weights per sample: wx[8] wy[8] (wz[8])
+  using TG = TileGeo<T>;
+  constexpr int CELLS = TG::CELLS, PY = TG::PY;
+  constexpr int WROW = 16;                 // staged weights per sample: wx[8] wy[8]
   extern __shared__ __align__(16) int smi[];
   __shared__ unsigned vmax[16];
   __shared__ float scale[16], inv_scale[16];
@@ -594,11 +587,7 @@ __global__ void __launch_bounds__(256) k_spread(NufftGeom g, TileShape t, const 
   const int tile = sp.x, first = sp.z, count = sp.w;
   const int lseg = sp.y;
   if (!PG_CHECK(count <= smax, PG_SITE_SPREAD_COUNT, count)) continue;   // uniform across the block
-  const int ty = tile % t.nty;
-  const int txz = tile / t.nty;
-  const int tx = txz % t.ntx;
-  const int tz = txz / t.ntx;
-  const int x0 = tx * T, y0 = ty * T, z0 = tz * TG::TZ;
+  const int x0 = (tile / t.nty) * T, y0 = (tile % t.nty) * T;
   const int tid = threadIdx.x;
   float* sw = reinterpret_cast<float*>(smi + (size_t)np * 2 * CELLS);
   float2* sv = reinterpret_cast<float2*>(sw + (size_t)smax * WROW);
@@ -609,9 +598,8 @@ __global__ void __launch_bounds__(256) k_spread(NufftGeom g, TileShape t, const 
   constexpr int R4 = WROW / 4;
   for (int q = tid; q < count * R4; q += blockDim.x) {
     const int i = q / R4, a = q % R4;
-    const float4* src = (a < 4) ? reinterpret_cast<const float4*>(wxy + (uint64_t)(first + i) * 16) + a
-                                : reinterpret_cast<const float4*>(wz + (uint64_t)(first + i) * 8) + (a - 4);
-    cp_async16(reinterpret_cast<float4*>(sw + i * WROW) + a, src);
+    cp_async16(reinterpret_cast<float4*>(sw + i * WROW) + a,
+               reinterpret_cast<const float4*>(wxy + (uint64_t)(first + i) * 16) + a);
   }
   for (int i = tid; i < count; i += blockDim.x) cp_async8(&sst[i], &start[first + i]);
   // sv[i][c*K + j] = vs[cfirst + c][first + i][j]: for each coil of the block
@@ -660,7 +648,7 @@ __global__ void __launch_bounds__(256) k_spread(NufftGeom g, TileShape t, const 
   const int warp = tid >> 5, lane = tid & 31;
   constexpr int NW = 8;
   const int dy = lane & 7, dx = lane >> 3;
-  if (DIM == 2 && NP > 0) {
+  if (NP > 0) {
     // Each warp walks a contiguous run of samples.  Samples are in readout
     // order within a bin, so consecutive ones often share their window start;
     // a lane then keeps hitting the same two cells, so it sums the run's
@@ -721,44 +709,22 @@ __global__ void __launch_bounds__(256) k_spread(NufftGeom g, TileShape t, const 
     for (int i = warp; i < count; i += NW) {
       const uint2 st = sst[i];
       const int ox = (int)(st.x & 0xffff) - x0, oy = (int)(st.x >> 16) - y0;
-      if (!PG_CHECK(ox >= 0 && ox < T && oy >= 0 && oy < T &&
-                        (DIM == 2 || ((int)st.y - z0 >= 0 && (int)st.y - z0 < TG::TZ)),
-                    PG_SITE_SPREAD_WINDOW, ox * 65536 + oy))
+      if (!PG_CHECK(ox >= 0 && ox < T && oy >= 0 && oy < T, PG_SITE_SPREAD_WINDOW, ox * 65536 + oy))
         continue;                          // uniform across the warp
       const float* w = sw + i * WROW;
       const float wyv = w[8 + dy];
       const float w0 = w[dx] * wyv, w1 = w[dx + 4] * wyv;
       int* b = smi + (ox + dx) * PY + oy + dy;
       const float2* vi = sv + i * np;
-      if (DIM == 2) {
 #pragma unroll
-        for (int pl = 0; pl < np; ++pl) {
-          const float2 u = vi[pl];
-          const float sc = scale[pl];
-          const float2 v = make_float2(u.x * sc, u.y * sc);
-          atomicAdd(b + (2 * pl) * CELLS, fixed_point(w0, v.x));
-          atomicAdd(b + (2 * pl + 1) * CELLS, fixed_point(w0, v.y));
-          atomicAdd(b + (2 * pl) * CELLS + 4 * PY, fixed_point(w1, v.x));
-          atomicAdd(b + (2 * pl + 1) * CELLS + 4 * PY, fixed_point(w1, v.y));
-        }
-      } else {
-        b += ((int)st.y - z0) * PLANE;
-#pragma unroll 1
-        for (int e = 0; e < 8; ++e, b += PLANE) {
-          const float wzv = w[16 + e];
-          if (wzv == 0.f) continue;          // uniform across the warp
-          const float w0e = w0 * wzv, w1e = w1 * wzv;
-#pragma unroll
-          for (int pl = 0; pl < np; ++pl) {
-            const float2 u = vi[pl];
-            const float sc = scale[pl];
-            const float2 v = make_float2(u.x * sc, u.y * sc);
-            atomicAdd(b + (2 * pl) * CELLS, fixed_point(w0e, v.x));
-            atomicAdd(b + (2 * pl + 1) * CELLS, fixed_point(w0e, v.y));
-            atomicAdd(b + (2 * pl) * CELLS + 4 * PY, fixed_point(w1e, v.x));
-            atomicAdd(b + (2 * pl + 1) * CELLS + 4 * PY, fixed_point(w1e, v.y));
-          }
-        }
+      for (int pl = 0; pl < np; ++pl) {
+        const float2 u = vi[pl];
+        const float sc = scale[pl];
+        const float2 v = make_float2(u.x * sc, u.y * sc);
+        atomicAdd(b + (2 * pl) * CELLS, fixed_point(w0, v.x));
+        atomicAdd(b + (2 * pl + 1) * CELLS, fixed_point(w0, v.y));
+        atomicAdd(b + (2 * pl) * CELLS + 4 * PY, fixed_point(w1, v.x));
+        atomicAdd(b + (2 * pl + 1) * CELLS + 4 * PY, fixed_point(w1, v.y));
       }
     }
   }
@@ -767,12 +733,9 @@ __global__ void __launch_bounds__(256) k_spread(NufftGeom g, TileShape t, const 
   // 4. flush
   const uint64_t G = g.ngrid();
   for (int q = tid; q < CELLS; q += blockDim.x) {
-    const int pyy = q % PY;
-    const int pxx = (q / PY) % PX;
-    const int pzz = q / PLANE;
-    const int gy = y0 + pyy, gx = x0 + pxx, gz = z0 + pzz;
-    const bool inside = gy < g.Gy && gx < g.Gx && gz < g.Gz;
-    const uint64_t idx = (uint64_t)gy + (uint64_t)g.Gy * ((uint64_t)gx + (uint64_t)g.Gx * gz);
+    const int gy = y0 + q % PY, gx = x0 + q / PY;
+    const bool inside = gy < g.Gy && gx < g.Gx;
+    const uint64_t idx = (uint64_t)gy + (uint64_t)g.Gy * (uint64_t)gx;
     int pl = 0;
     for (int c = 0; c < cc; ++c)
       for (int j = 0; j < K; ++j, ++pl) {
@@ -829,7 +792,7 @@ __global__ void __launch_bounds__(256, spread2d_min_blocks(CC * KK))
                                                   int smax, float wmax, float2* __restrict__ grids,
                                                   unsigned* __restrict__ queue, int nchunks, int nitems) {
   pdl_wait();
-  using TG = TileGeo<2, T>;
+  using TG = TileGeo<T>;
   constexpr int CELLS = TG::CELLS, PY = TG::PY;
   constexpr int NP = CC * KK;          // planes per item
   constexpr int NP2 = (NP + 1) / 2;    // 16-byte value slots per sample
@@ -1694,7 +1657,7 @@ static pg_status ensure_queue(NufftPlan* p, cudaStream_t s) {
 template <int T, int CC, int KP>
 static pg_status gather_launch_one(NufftPlan* p, const Binning* bin, const float2* aa, int nb, float2* y,
                                    uint64_t dstride, cudaStream_t s) {
-  const size_t smem = (size_t)CC * KP * 2 * TileGeo<2, T>::CELLS * sizeof(float);
+  const size_t smem = (size_t)CC * KP * 2 * TileGeo<T>::CELLS * sizeof(float);
   PG_CUDA(cudaFuncSetAttribute(k_gather<T, CC, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // a static grid: the persistent work-queue form measured ~4 % slower here
   dim3 grid(bin->nsub * 2, ceil_div(nb, CC));
@@ -1708,7 +1671,7 @@ static pg_status launch_gather_t(NufftPlan* p, const Binning* bin, const float2*
                                  uint64_t dstride, cudaStream_t s) {
   const int K = bin->K;
   const int KP = K <= 1 ? 1 : K <= 2 ? 2 : K <= 4 ? 4 : 8;
-  const size_t pair = (size_t)TileGeo<2, T>::CELLS * 2 * sizeof(float);
+  const size_t pair = (size_t)TileGeo<T>::CELLS * 2 * sizeof(float);
   const size_t limit = (size_t)smem_optin_bytes() - 6144;  // static reduction buffer + margin
   int CC = std::max(1, std::min(4, p->tune.gather_cc));
   while (CC > 1 && (CC >= 2 * nb || 2 * CC * KP > 32 || (size_t)CC * KP * pair > limit)) CC >>= 1;
@@ -1779,39 +1742,39 @@ struct SpreadArgs {
   size_t smem;
 };
 
-template <int DIM, int T, int NP>
+template <int T, int NP>
 static pg_status spread_launch_np(NufftPlan* p, const Binning* bin, const SpreadArgs& a, float2* target,
                                   cudaStream_t s) {
-  PG_TRY(allow_full_dynamic_smem((const void*)k_spread<DIM, T, NP>));
+  PG_TRY(allow_full_dynamic_smem((const void*)k_spread<T, NP>));
   const int nitems = bin->nsub * a.nchunks;
   PG_TRY(ensure_queue(p, s));
-  const int blocks = persistent_blocks((const void*)k_spread<DIM, T, NP>, a.smem, nitems);
-  PG_LAUNCH_PDL((k_spread<DIM, T, NP>), blocks, 256, a.smem, s, p->g, bin->tile, bin->subprob.p, bin->start.p,
-            bin->wxy.p, bin->wz.p, a.vs, bin->M, bin->K, bin->L, a.c0, a.cc, bin->submax, a.wmax, target,
+  const int blocks = persistent_blocks((const void*)k_spread<T, NP>, a.smem, nitems);
+  PG_LAUNCH_PDL((k_spread<T, NP>), blocks, 256, a.smem, s, p->g, bin->tile, bin->subprob.p, bin->start.p,
+            bin->wxy.p, a.vs, bin->M, bin->K, bin->L, a.c0, a.cc, bin->submax, a.wmax, target,
             p->work->queue.p, a.nchunks, nitems);
   return PG_OK;
 }
 
 // Planes per block (coils x segments) with an unrolled kernel; others use the
 // runtime-loop instantiation (NP = 0).
-template <int DIM, int T>
+template <int T>
 static pg_status spread_launch_t(NufftPlan* p, const Binning* bin, const SpreadArgs& a, float2* target,
                                  cudaStream_t s) {
   switch (a.cc * bin->K) {
-    case 1: return spread_launch_np<DIM, T, 1>(p, bin, a, target, s);
-    case 2: return spread_launch_np<DIM, T, 2>(p, bin, a, target, s);
-    case 3: return spread_launch_np<DIM, T, 3>(p, bin, a, target, s);
-    case 4: return spread_launch_np<DIM, T, 4>(p, bin, a, target, s);
-    case 6: return spread_launch_np<DIM, T, 6>(p, bin, a, target, s);
-    case 8: return spread_launch_np<DIM, T, 8>(p, bin, a, target, s);
+    case 1: return spread_launch_np<T, 1>(p, bin, a, target, s);
+    case 2: return spread_launch_np<T, 2>(p, bin, a, target, s);
+    case 3: return spread_launch_np<T, 3>(p, bin, a, target, s);
+    case 4: return spread_launch_np<T, 4>(p, bin, a, target, s);
+    case 6: return spread_launch_np<T, 6>(p, bin, a, target, s);
+    case 8: return spread_launch_np<T, 8>(p, bin, a, target, s);
   }
-  return spread_launch_np<DIM, T, 0>(p, bin, a, target, s);
+  return spread_launch_np<T, 0>(p, bin, a, target, s);
 }
 
 static pg_status launch_spread(NufftPlan* p, const Binning* bin, const SpreadArgs& a, float2* target,
                                cudaStream_t s) {
-  if (bin->tile.TX == 32) return spread_launch_t<2, 32>(p, bin, a, target, s);
-  return spread_launch_t<2, 16>(p, bin, a, target, s);
+  if (bin->tile.TX == 32) return spread_launch_t<32>(p, bin, a, target, s);
+  return spread_launch_t<16>(p, bin, a, target, s);
 }
 
 // Shared memory of k_spread2d: tile planes, staged weights, values and starts.
@@ -1970,7 +1933,7 @@ pg_status nufft_adjoint(NufftPlan* p, const NufftBatch& b, const float2* y, floa
   const int smax = bin->submax;
   // tile planes of cc coils x K segments, plus the staged samples
   auto smem_for = [&](int cc) {
-    return plane_bytes * K * cc + (size_t)smax * (spread_wrow(g.dim) * sizeof(float) + sizeof(uint2) +
+    return plane_bytes * K * cc + (size_t)smax * (16 * sizeof(float) + sizeof(uint2) +
                                                   (size_t)K * cc * sizeof(float2));
   };
   // 3-D, and 2-D with K <= 2 (Hanning segments or none): the spread reads the
@@ -2051,7 +2014,9 @@ pg_status nufft_adjoint(NufftPlan* p, const NufftBatch& b, const float2* y, floa
     }
     }
     }
-    const int acc = (b.accumulate || c0 > 0) ? 1 : 0;
+    // a later batch adds to the image of an earlier one; with several images the
+    // passes know which of them began earlier
+    const int acc = (b.accumulate || (c0 > 0 && b.cgroup == 0)) ? 1 : 0;
     if (p->own_fft) {
       PG_TRY(grow(p->work->fin, fftpass_scratch(g, B), s));
       const FftBatch fb{nb, L, c0, b.S, b.E, b.cgroup, b.image_stride, b.phase_stride};

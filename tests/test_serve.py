@@ -130,6 +130,35 @@ def test_batched_slices_match_per_slice_solves(pg, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [256, 250])
+def test_batched_slices_split_over_workspace(pg, n):
+    """A job whose coils do not fit the grid workspace at once (2 GiB per job):
+    an image begins in one batch of coils and ends in the next, others begin in
+    a later batch.  Own FFT passes (256) and cuFFT (250)."""
+    from powergrid_b200 import synthetic as S
+    from powergrid_b200.serve import ReconRequest, Server
+    nc, L, ns, M = 20, 12, 5, 2048
+    kx, ky, t = S.spiral(n, 2, M // 2, 10e-3)
+    kz = np.zeros_like(kx)
+    fm = np.stack([S.field_map(S.Rng(60 + s), n, n, 1, 80.0) for s in range(ns)])
+    sm = np.stack([S.coil_maps(S.Rng(70 + s), n, n, 1, nc) for s in range(ns)])
+    y = np.stack([S.image(S.Rng(80 + s), M * nc) for s in range(ns)])
+
+    def req(sl):
+        k = len(sl)
+        return ReconRequest(n, n, 1, nc, L, 2, 1e-3, kx, ky, kz, t, fm[sl], sm[sl].ravel(), y[sl].ravel(), k)
+
+    srv = Server(hbm_budget_bytes=40 << 30, max_inflight=1)
+    img, st = srv.wait(srv.submit(req(list(range(ns)))))
+    assert st["status"] == "PG_OK" and st["jobs"] == 1
+    for s in range(ns):
+        one, st = srv.wait(srv.submit(req([s])))
+        assert st["status"] == "PG_OK"
+        assert rel_l2(img[s], one[0]) <= MIX_TOL
+    srv.close()
+
+
+@pytest.mark.gpu
 def test_admission_rejects_oversized_request(pg):
     from powergrid_b200 import synthetic as S
     from powergrid_b200._lib import PGError
