@@ -4,9 +4,13 @@
 //   forward  y_i = sum_j x_j exp(-i (2pi k_i . r_j + FM_j t_i))
 //   adjoint  x_j = sum_i y_i exp(+i (2pi k_i . r_j + FM_j t_i))
 // The reference evaluates the phase and sinf/cosf in FP32.  Here the phase
-// is formed with FP64 products and reduced mod 2pi in FP64, then one FP32
-// __sincosf serves every coil of the pair; the complex MACs are FP32 with a
-// two-level (per-tile, then running) sum.
+// is formed in turns with FP64 products and reduced mod 1 in FP64, then one
+// FP32 __sincosf serves every coil of the pair.
+//
+// Two sets of kernels.  From kTensorCoils coils on, the sums over the pairs run
+// on the tensor cores (pg_gdft_tc.cu); below that, and for plans whose phases
+// its fixed-point form cannot hold, here: complex MACs in FP32 with a two-level
+// (per-tile, then running) sum.
 //
 // GdftR2 (ftCpuWithGrads.cpp:93-216) multiplies each pair by
 //   sinc(kx_i/Nx + Gx_j t_i) sinc(ky_i/Ny + Gy_j t_i) sinc(kz_i/Nz + Gz_j t_i),
@@ -20,9 +24,11 @@
 // combined once per tile (forward A - iB, adjoint A + iB).  When the
 // outputs alone do not fill the GPU the inner sum is split over blockIdx.y
 // and the partial sums are combined in a fixed order (deterministic).
+#include <algorithm>
 #include <vector>
 
 #include "pg_gdft.cuh"
+#include "pg_gdft_tc.cuh"
 #include "pg_profile.cuh"
 
 namespace pg {
@@ -42,16 +48,14 @@ __device__ __forceinline__ float grad_factor(float4 kn, float4 gm) {
   return sinc_pg(kn.x + gm.x * kn.w) * sinc_pg(kn.y + gm.y * kn.w) * sinc_pg(kn.z + gm.z * kn.w);
 }
 
+// sin and cos of 2 pi ph, ph in turns.
 __device__ __forceinline__ void phase_sincos(double ph, float* s, float* c) {
-  const double inv2pi = 0.15915494309189533577;   // 1 / (2 pi)
-  const double twopi = 6.283185307179586476925;    // 2 pi (double)
-  const double n = rint(ph * inv2pi);
-  const float r = (float)fma(-n, twopi, ph);      // |r| <= pi
+  const float r = (float)((ph - rint(ph)) * 6.283185307179586476925);   // |r| <= pi
   __sincosf(r, s, c);
 }
 }  // namespace
 
-// Forward partial sums.  ks[i] = (2pi kx, 2pi ky, 2pi kz, t); vs[j] = (ix, iy, iz, FM).
+// Forward partial sums.  ks[i] = (kx, ky, kz, t / 2 pi); vs[j] = (ix, iy, iz, FM).
 // xin: nc x ni inputs (already multiplied by the coil maps).
 template <int NC, bool GRAD>
 __global__ void __launch_bounds__(kTile) k_dft_forward(uint64_t nk, uint64_t ni, const double4* __restrict__ ks,
@@ -217,6 +221,13 @@ __global__ void k_adjoint_finish(uint64_t ni, int nc, int c0, int nsplit, int nc
 static pg_status upload_samples(GdftPlan* p, uint64_t nk, const float* kx, const float* ky, const float* kz,
                                 const float* t, cudaStream_t s);
 
+static void widen(double (&m)[4], const double4& v) {
+  m[0] = std::max(m[0], std::abs(v.x));
+  m[1] = std::max(m[1], std::abs(v.y));
+  m[2] = std::max(m[2], std::abs(v.z));
+  m[3] = std::max(m[3], std::abs(v.w));
+}
+
 pg_status gdft_plan_create(std::unique_ptr<GdftPlan>* out, uint64_t nk, uint64_t ni, const float* kx, const float* ky,
                            const float* kz, const float* ix, const float* iy, const float* iz, const float* fm,
                            const float* t, cudaStream_t s) {
@@ -224,13 +235,14 @@ pg_status gdft_plan_create(std::unique_ptr<GdftPlan>* out, uint64_t nk, uint64_t
   auto p = std::make_unique<GdftPlan>();
   p->nk = nk;
   p->ni = ni;
-  std::vector<double4> vs(ni);
+  std::vector<double4> vs(gdft_tc_padded(ni), make_double4(0, 0, 0, 0));
   for (uint64_t j = 0; j < ni; ++j) {
     if (!(std::isfinite(ix[j]) && std::isfinite(iy[j]) && std::isfinite(iz[j]) && std::isfinite(fm[j])))
       return set_error(PG_INVALID_ARG, "Gdft: non-finite voxel input at %llu", (unsigned long long)j);
     vs[j] = make_double4(ix[j], iy[j], iz[j], fm[j]);
+    widen(p->vmax, vs[j]);
   }
-  PG_TRY(p->vs.upload(vs.data(), ni, s));
+  PG_TRY(p->vs.upload(vs.data(), vs.size(), s));
   PG_TRY(upload_samples(p.get(), nk, kx, ky, kz, t, s));
   *out = std::move(p);
   return PG_OK;
@@ -239,13 +251,18 @@ pg_status gdft_plan_create(std::unique_ptr<GdftPlan>* out, uint64_t nk, uint64_t
 static pg_status upload_samples(GdftPlan* p, uint64_t nk, const float* kx, const float* ky, const float* kz,
                                 const float* t, cudaStream_t s) {
   const double tpi = 6.283185307179586476925;
-  std::vector<double4> ks(nk);
+  std::vector<double4> ks(gdft_tc_padded(nk), make_double4(0, 0, 0, 0));
+  double kmax[4] = {0, 0, 0, 0};
   for (uint64_t i = 0; i < nk; ++i) {
     if (!(std::isfinite(kx[i]) && std::isfinite(ky[i]) && std::isfinite(kz[i]) && std::isfinite(t[i])))
       return set_error(PG_INVALID_ARG, "Gdft: non-finite sample input at %llu", (unsigned long long)i);
-    ks[i] = make_double4(tpi * kx[i], tpi * ky[i], tpi * kz[i], (double)t[i]);
+    ks[i] = make_double4(kx[i], ky[i], kz[i], (double)t[i] / tpi);
+    widen(kmax, ks[i]);
   }
-  PG_TRY(p->ks.upload(ks.data(), nk, s));
+  double bound = 0.0;
+  for (int a = 0; a < 4; ++a) bound += kmax[a] * p->vmax[a];
+  p->turns_fit = bound < kTurnLimit;
+  PG_TRY(p->ks.upload(ks.data(), ks.size(), s));
   PG_CUDA(cudaStreamSynchronize(s));
   return PG_OK;
 }
@@ -257,6 +274,7 @@ pg_status gdft_plan_same_voxels(std::unique_ptr<GdftPlan>* out, const GdftPlan& 
   p->nk = nk;
   p->ni = src.ni;
   p->vs.borrow(src.vs);
+  std::copy(src.vmax, src.vmax + 4, p->vmax);
   p->work = src.work;
   PG_TRY(upload_samples(p.get(), nk, kx, ky, kz, t, s));
   *out = std::move(p);
@@ -282,12 +300,12 @@ pg_status gdft_plan_add_gradients(GdftPlan* p, const float* kx, const float* ky,
   cd(1, &gx);
   cd((uint64_t)ny, &gy);
   cd((uint64_t)nx * ny, &gz);
-  std::vector<float4> gm(N), kn(p->nk);
+  std::vector<float4> gm(gdft_tc_padded(N), make_float4(0.f, 0.f, 0.f, 0.f)), kn(gdft_tc_padded(p->nk), gm[0]);
   for (uint64_t j = 0; j < N; ++j) gm[j] = make_float4(gx[j], gy[j], gz[j], 0.f);
   for (uint64_t i = 0; i < p->nk; ++i)
     kn[i] = make_float4(kx[i] / (float)nx, ky[i] / (float)ny, kz[i] / (float)nz, t[i]);
-  PG_TRY(p->gm.upload(gm.data(), N, s));
-  PG_TRY(p->kn.upload(kn.data(), p->nk, s));
+  PG_TRY(p->gm.upload(gm.data(), gm.size(), s));
+  PG_TRY(p->kn.upload(kn.data(), kn.size(), s));
   PG_CUDA(cudaStreamSynchronize(s));
   return PG_OK;
 }
@@ -327,10 +345,40 @@ static pg_status launch_adj(GdftPlan* p, int nsplit, uint64_t ichunk, const floa
   return PG_OK;
 }
 
+// Where the tensor cores' sums are the faster ones.  Their cost does not depend
+// on the number of coils up to 8 (then up to 16): at 64^2 x 32, 131072 samples,
+// 8 coils 20.7 ms against 34.5 ms; 47^2 x 8, 56544 samples, 13 coils with gradients
+// 6.8 against 13.3 ms; 36^2 x 11, 2 x 11231 samples, 3 coils, both directions 0.95
+// against 1.14 ms.  With 1 or 2 coils the plain kernels have the fewer
+// instructions per pair.  Small sums do not make up for the packing launches and
+// the start of a CTA: 2304 voxels x 1636 samples, 6 coils, 4 shots, both
+// directions 418 against 397 us.
+constexpr int kTensorCoils = 3;
+constexpr uint64_t kTensorPairs = 1ull << 25;
+
+static bool use_tensor(const GdftPlan& p, int C) {
+  return p.turns_fit && C >= kTensorCoils && p.nk * p.ni >= kTensorPairs;
+}
+
 static int pad_coils(int nc) { return nc <= 1 ? 1 : nc <= 2 ? 2 : nc <= 4 ? 4 : 8; }
 
 pg_status gdft_forward(GdftPlan* p, int C, const float2* S, const float2* x, float2* y, uint64_t dstride,
                        cudaStream_t s) {
+  if (use_tensor(*p, C)) {
+    const GdftSide g{p->nk, p->ni, p->ks.p, p->vs.p, p->kn.p, p->gm.p, true};
+    const int ncp = gdft_tc_coils(C), ns = gdft_tc_splits(p->nk, p->ni, ncp);
+    PG_TRY(grow(p->work->B, gdft_tc_operand(p->ni, ncp), s));
+    PG_TRY(grow(p->work->part, (uint64_t)ns * ncp * p->nk, s));
+    for (int c0 = 0; c0 < C; c0 += ncp) {
+      const int nc = std::min(ncp, C - c0);
+      PG_TRY(gdft_tc_pack(g, nc, ncp, S ? S + (uint64_t)c0 * p->ni : nullptr, x, 0, p->work->B.p, s));
+      ProfScope ps("dft_fwd", s);
+      PG_TRY(gdft_tc_sum(g, ncp, ns, p->work->B.p, p->work->part.p, s));
+      PG_LAUNCH(k_forward_finish, ceil_div(p->nk, 256), 256, 0, s, p->nk, nc, ns, ncp, p->work->part.p,
+                y + (uint64_t)c0 * dstride, dstride);
+    }
+    return PG_OK;
+  }
   const int nsplit = splits_for(p->nk, p->ni);
   uint64_t jchunk = (p->ni + nsplit - 1) / nsplit;
   jchunk = (jchunk + kTile - 1) / kTile * kTile;
@@ -356,6 +404,21 @@ pg_status gdft_forward(GdftPlan* p, int C, const float2* S, const float2* x, flo
 
 pg_status gdft_adjoint(GdftPlan* p, int C, const float2* S, const float2* y, uint64_t dstride, float2* x,
                        cudaStream_t s) {
+  if (use_tensor(*p, C)) {
+    const GdftSide g{p->ni, p->nk, p->vs.p, p->ks.p, p->gm.p, p->kn.p, false};
+    const int ncp = gdft_tc_coils(C), ns = gdft_tc_splits(p->ni, p->nk, ncp);
+    PG_TRY(grow(p->work->B, gdft_tc_operand(p->nk, ncp), s));
+    PG_TRY(grow(p->work->part, (uint64_t)ns * ncp * p->ni, s));
+    for (int c0 = 0; c0 < C; c0 += ncp) {
+      const int nc = std::min(ncp, C - c0);
+      PG_TRY(gdft_tc_pack(g, nc, ncp, nullptr, y + (uint64_t)c0 * dstride, dstride, p->work->B.p, s));
+      ProfScope ps("dft_adj", s);
+      PG_TRY(gdft_tc_sum(g, ncp, ns, p->work->B.p, p->work->part.p, s));
+      PG_LAUNCH(k_adjoint_finish, ceil_div(p->ni, 256), 256, 0, s, p->ni, nc, c0, ns, ncp, p->work->part.p, S,
+                c0 > 0 ? 1 : 0, x);
+    }
+    return PG_OK;
+  }
   const int nsplit = splits_for(p->ni, p->nk);
   uint64_t ichunk = (p->nk + nsplit - 1) / nsplit;
   ichunk = (ichunk + kTile - 1) / kTile * kTile;

@@ -8,19 +8,24 @@
 
 namespace pg {
 
-// Staged coil inputs and split partial sums.  Plans applied one after
+// Staged coil inputs, packed tensor-core operand and split partial sums.  Plans applied one after
 // another on one stream (the shots of pcSENSE) share a single one.
 struct GdftWork {
   DevBuf<float2> xin;
+  DevBuf<uint32_t> B;
   DevBuf<float2> part;
 };
 
 struct GdftPlan {
   uint64_t nk = 0, ni = 0;
-  DevBuf<double4> ks;    // per sample (2pi kx, 2pi ky, 2pi kz, t)
+  // the pair's phase in turns is the product of these two (k.r + FM t / 2 pi);
+  // both padded with zeros to whole tensor-core tiles
+  DevBuf<double4> ks;    // per sample (kx, ky, kz, t / 2 pi)
   DevBuf<double4> vs;    // per voxel (ix, iy, iz, FM rad/s); may view another plan's
+  double vmax[4] = {0, 0, 0, 0};   // largest magnitudes of vs
+  bool turns_fit = false;          // every phase is below kTurnLimit turns
   std::shared_ptr<GdftWork> work = std::make_shared<GdftWork>();
-  // GdftR2 only: per sample (kx/Nx, ky/Ny, kz/Nz, t), per voxel (Gx, Gy, Gz, 0)
+  // GdftR2 only: per sample (kx/Nx, ky/Ny, kz/Nz, t), per voxel (Gx, Gy, Gz, 0), padded like ks, vs
   DevBuf<float4> kn;
   DevBuf<float4> gm;
 };
