@@ -22,6 +22,8 @@
 
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "pg_fftdft.cuh"
 #include "pg_fftpass.cuh"
 
@@ -52,6 +54,7 @@ struct FftRows {
   const uint32_t* rows;             // support words [segment][R1]
   const float2* tw;
   int split;                        // forward: blocks per coil; inverse: blocks per image
+  int cluster;                      // inverse: the blocks of an image are a cluster
 };
 
 struct FftOps {
@@ -59,13 +62,21 @@ struct FftOps {
   pg_status (*rows_fwd)(const NufftGeom& g, const FftRows& a, const float2* x, float2* P, cudaStream_t s);
   pg_status (*cols_fwd)(const FftLines& a, uint64_t nsets, const float2* in, float2* out, cudaStream_t s);
   pg_status (*cols_inv)(const FftLines& a, uint64_t nsets, float2* in, int clear, float2* out, cudaStream_t s);
-  // out: `split` partial images per image, or (split == 1) x itself
+  // out: x, or partial images (split > 1 without a cluster)
   pg_status (*rows_inv)(const NufftGeom& g, const FftRows& a, int nimages, const float2* Q, int accumulate,
                         float2* out, cudaStream_t s);
-  int rows_per_block;
+  int rows_per_block, row_blocks_per_sm;
+  // both in-plane passes of a 2-D grid in one block per grid, or null
+  pg_status (*grid_fwd)(const NufftGeom& g, const FftRows& a, const uint32_t* xmask, const float2* x, float2* grids,
+                        cudaStream_t s);
+  // split: the grids of an image; out: x, or every grid's image (split > 1 without a cluster)
+  pg_status (*grid_inv)(const NufftGeom& g, const FftRows& a, const uint32_t* xmask, float2* grids, int clear,
+                        int accumulate, float2* out, cudaStream_t s);
 };
 
 namespace fftk {
+
+namespace cg = cooperative_groups;
 
 __host__ __device__ constexpr int imax(int a, int b) { return a > b ? a : b; }
 __host__ __device__ constexpr int imin(int a, int b) { return a < b ? a : b; }
@@ -78,6 +89,10 @@ struct RowGeo {
   static constexpr int n = R1 * R2;
   static constexpr int RB = n >= 1024 ? 4 : imax(R1, R2) > 16 ? 8 : 16;
   static constexpr int T = (RB * imax(R1, R2) + 31) / 32 * 32;
+  // blocks per SM the registers are held to: the passes wait for memory between
+  // their two barriers per grid (96^2 x 16, 8 coils, L = 6: last inverse pass with
+  // its summing 94 -> 50 us; 208^2, 12 coils, L = 10: 62 -> 53 us)
+  static constexpr int MINB = imax(R1, R2) <= 16 ? imin(4, 768 / T) : 2;
 };
 // Shared layout [row][k1 < RA][m2 < RBk]: odd m2 stride (the second pass's
 // threads, one k1 each, hit distinct banks), row stride = RBk (mod 16).
@@ -107,7 +122,7 @@ __device__ __forceinline__ int parity2(int a, int b) { return (a + b) & 1; }
 // per segment of the block's share the phase Wo and the FFT along y of the
 // zero-padded line -> P[c * L + l][iz][ix][0..n), supported groups only.
 template <int R1, int R2>
-__global__ void __launch_bounds__((RowGeo<R1, R2>::T)) k_fft_fwd_rows(NufftGeom g, FftRows a,
+__global__ void __launch_bounds__((RowGeo<R1, R2>::T), (RowGeo<R1, R2>::MINB)) k_fft_fwd_rows(NufftGeom g, FftRows a,
                                                                       const float2* __restrict__ x,
                                                                       float2* __restrict__ P) {
   pdl_wait();
@@ -146,18 +161,27 @@ __global__ void __launch_bounds__((RowGeo<R1, R2>::T)) k_fft_fwd_rows(NufftGeom 
     }
   }
   const float2* W = a.W ? a.W + (uint64_t)img * a.phase_stride : nullptr;
+  float2 w[H];
+  if (W && in_a) {
+#pragma unroll
+    for (int h = 0; h < H; ++h) w[h] = W[(uint64_t)l0 * N + p0 + R2 * h];
+  }
   for (int l = l0; l < l1; ++l) {
     if (in_a) {
       float2 v[R1];
 #pragma unroll
       for (int m1 = 0; m1 < R1; ++m1) v[m1] = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int h = 0; h < H; ++h) v[R1 / 4 + h] = W ? cmul(W[(uint64_t)l * N + p0 + R2 * h], u[h]) : u[h];
+      for (int h = 0; h < H; ++h) v[R1 / 4 + h] = W ? cmul(w[h], u[h]) : u[h];
       dft<R1>(v, false);
       float2* d = sh + ra * SM::RS + m2;
       d[0] = v[0];
 #pragma unroll
       for (int q = 1; q < R1; ++q) d[q * SM::S2] = twiddle(v[q], a.tw[q * R2 + m2], false);
+      if (W && l + 1 < l1) {               // the next segment's phases arrive during the second pass
+#pragma unroll
+        for (int h = 0; h < H; ++h) w[h] = W[(uint64_t)(l + 1) * N + p0 + R2 * h];
+      }
     }
     __syncthreads();
     if (in_b) {
@@ -278,9 +302,13 @@ __global__ void __launch_bounds__((ColGeo<R1, R2>::T)) k_fft_inv_cols(FftLines a
 #pragma unroll
     for (int q = 1; q < R2; ++q) d[q * S1] = twiddle(v[q], tw[q * R1 + m2], true);
     if constexpr (CLEAR) {
+      // the addresses anew: kept from the loads they took up to 180 registers
+      // (208^2, 12 coils, L = 10: 63 -> 45 us)
+      uint64_t oc = o;
+      asm volatile("" : "+l"(oc));
 #pragma unroll
       for (int m1 = 0; m1 < R2; ++m1)
-        if (sup >> m1 & 1u) inw[o + (uint64_t)(R1 * m1) * a.rstride] = make_float2(0.f, 0.f);
+        if (sup >> m1 & 1u) inw[oc + (uint64_t)(R1 * m1) * a.rstride] = make_float2(0.f, 0.f);
     }
   }
   __syncthreads();
@@ -306,11 +334,12 @@ __global__ void __launch_bounds__((ColGeo<R1, R2>::T)) k_fft_inv_cols(FftLines a
 
 // Last inverse pass: lines (ix, iz) of the block's share of an image's grids,
 // inverse FFT along y, crop, WoH, conj coil map and conj shot phase, summed
-// over the share in grid order in registers; deapodization and sign once at
-// the end.  One partial image per share (or the image itself for one share):
-// the grids' images never reach memory.
+// over the share in grid order in registers; shot phase, deapodization and sign
+// once at the end.  Up to 8 shares of one group of lines are the blocks of a cluster,
+// which adds them in rank order through distributed shared memory; more shares
+// (small images, which need them to fill the GPU) write partial images.
 template <int R1, int R2>
-__global__ void __launch_bounds__((RowGeo<R1, R2>::T)) k_fft_inv_rows(NufftGeom g, FftRows a, int nimages,
+__global__ void __launch_bounds__((RowGeo<R1, R2>::T), (RowGeo<R1, R2>::MINB)) k_fft_inv_rows(NufftGeom g, FftRows a, int nimages,
                                                                       const float2* __restrict__ Q, int accumulate,
                                                                       float2* __restrict__ out) {
   pdl_wait();
@@ -336,9 +365,9 @@ __global__ void __launch_bounds__((RowGeo<R1, R2>::T)) k_fft_inv_rows(NufftGeom 
   const uint64_t p0 = (uint64_t)k1 + (uint64_t)Nn * (r0 + rb);
   const float2* W = a.W ? a.W + (uint64_t)img * a.phase_stride : nullptr;
   const float2* tw = a.tw + n;             // transposed: [k1 < R2][m2 < R1]
-  float2 acc[H], coil[H];                  // over the share; over the current coil's segments
+  float2 acc[H];                           // over the share
 #pragma unroll
-  for (int h = 0; h < H; ++h) acc[h] = coil[h] = make_float2(0.f, 0.f);
+  for (int h = 0; h < H; ++h) acc[h] = make_float2(0.f, 0.f);
   for (int b = b0; b < b1; ++b) {
     const int c = ca + b / a.L, l = b % a.L;
     if (in_a) {
@@ -363,40 +392,246 @@ __global__ void __launch_bounds__((RowGeo<R1, R2>::T)) k_fft_inv_rows(NufftGeom 
 #pragma unroll
       for (int q = 0; q < R1; ++q) u[q] = s[q];
       dft<R1>(u, true);
-      const bool last = l == a.L - 1 || b == b1 - 1;   // the coil's last segment here
 #pragma unroll
       for (int h = 0; h < H; ++h) {
+        const uint64_t p = p0 + R2 * h;
         float2 v = u[R1 / 4 + h];
-        if (W) v = cmul(v, W[(uint64_t)l * N + p0 + R2 * h]);
-        coil[h] = cadd(coil[h], v);
-      }
-      if (last) {
-#pragma unroll
-        for (int h = 0; h < H; ++h) {
-          float2 v = coil[h];
-          if (a.S) {
-            const float2 sv = cconj(a.S[(uint64_t)c * N + p0 + R2 * h]);
-            v = a.E ? cmul(cmul(sv, cconj(a.E[p0 + R2 * h])), v) : cmul(v, sv);
-          }
-          acc[h] = cadd(acc[h], v);
-          coil[h] = make_float2(0.f, 0.f);
-        }
+        if (W) v = cmul(v, W[(uint64_t)l * N + p]);
+        if (a.S) v = cmul(v, cconj(a.S[(uint64_t)c * N + p]));
+        acc[h] = cadd(acc[h], v);
       }
     }
     __syncthreads();
   }
-  if (!in_b) return;
-  const int rg = r0 + rb, ix = rg % g.Nx, iz = rg / g.Nx;
-  const int pxz = ix + g.crop_off[0] + iz + g.crop_off[2];
-  const bool add = a.split == 1 && (accumulate || (a.cgroup > 0 && img * a.cgroup < a.c0));
-  float2* o = a.split == 1 ? out + (uint64_t)img * a.image_stride : out + (uint64_t)is * N;
-#pragma unroll
-  for (int h = 0; h < H; ++h) {
-    const uint64_t p = p0 + R2 * h;
-    const float f = parity2(pxz, R2 * h + k1 + n / 4) ? -a.deapf[p] : a.deapf[p];
-    const float2 v = make_float2(acc[h].x * f, acc[h].y * f);
+  const bool partial = a.split > 1 && !a.cluster;
+  const bool add = !partial && (accumulate || (a.cgroup > 0 && img * a.cgroup < a.c0));
+  float2* o = partial ? out + (uint64_t)is * N : out + (uint64_t)img * a.image_stride;
+  auto store = [&](int row, int iy, float2 v) {
+    const int rg = r0 + row, pxz = rg % g.Nx + g.crop_off[0] + rg / g.Nx + g.crop_off[2];
+    const uint64_t p = (uint64_t)iy + (uint64_t)Nn * rg;
+    const float f = parity2(pxz, iy + n / 4) ? -a.deapf[p] : a.deapf[p];
+    if (a.S && a.E) v = cmul(cconj(a.E[p]), v);
+    v = make_float2(v.x * f, v.y * f);
     o[p] = add ? cadd(o[p], v) : v;
+  };
+  if (a.split == 1 || partial) {
+    if (in_b) {
+#pragma unroll
+      for (int h = 0; h < H; ++h) store(rb, k1 + R2 * h, acc[h]);
+    }
+    return;
   }
+  // every thread of every block of the cluster reaches both barriers
+  if (in_b) {
+#pragma unroll
+    for (int h = 0; h < H; ++h) sh[rb * Nn + k1 + R2 * h] = acc[h];
+  }
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  const int rows = min(RB, nrows - r0);
+  for (int i = part * RG::T + threadIdx.x; i < rows * Nn; i += a.split * RG::T) {
+    float2 v = *cl.map_shared_rank(sh + i, 0);
+    for (int q = 1; q < a.split; ++q) v = cadd(v, *cl.map_shared_rank(sh + i, q));
+    store(i / Nn, i % Nn, v);
+  }
+  cl.sync();   // no block leaves while another reads its shared memory
+}
+
+// ---------------------------------------------------------------------------
+// Small 2-D grids (n <= 64): both passes of a grid in one block, the half-
+// transformed rows in shared memory.  The values are those of the separate
+// passes.  At these sizes a pass is a few microseconds of latency over a handful
+// of blocks; one launch and one trip through L2 fewer per direction.  An operator
+// pair of 32 x 32, 2 coils, L = 4: 33.4 -> 28.2 us; at n = 128 one block per grid
+// was slower (a 64 x 64 solve of 3 steps 164 against 159 us).
+// ---------------------------------------------------------------------------
+template <int R1, int R2>
+struct GridGeo {
+  static constexpr int n = R1 * R2, N = n / 2;
+  static constexpr int T = 256;
+  static constexpr size_t held = (size_t)N * n;    // the transformed rows / the cropped columns
+  static constexpr size_t work = (size_t)imax(n * n, N * imax(RowSm<R1, R2>::RS, RowSm<R2, R1>::RS));
+  static constexpr size_t smem = (held + work) * sizeof(float2);
+};
+
+template <int R1, int R2>
+__global__ void __launch_bounds__((GridGeo<R1, R2>::T)) k_fft2_fwd_grid(NufftGeom g, FftRows a,
+                                                                       const uint32_t* __restrict__ xmask,
+                                                                       const float2* __restrict__ x,
+                                                                       float2* __restrict__ grids) {
+  pdl_wait();
+  using GG = GridGeo<R1, R2>;
+  using SM = RowSm<R1, R2>;
+  constexpr int n = GG::n, N = GG::N, T = GG::T, H = R1 / 2;
+  extern __shared__ float2 sh[];
+  float2* P = sh;                 // [row][n]
+  float2* Wk = sh + GG::held;
+  const int b = blockIdx.x, c = b / a.L, l = b - c * a.L, cg = a.c0 + c;
+  const int img = a.cgroup > 0 ? cg / a.cgroup : 0;
+  const float2* xi = x + (uint64_t)img * a.image_stride;
+  const float2* S = a.S ? a.S + (uint64_t)cg * N * N : nullptr;
+  const float2* W = a.W ? a.W + (uint64_t)img * a.phase_stride + (uint64_t)l * N * N : nullptr;
+  for (int it = threadIdx.x; it < N * R2; it += T) {         // y transform, first pass: (row, m2)
+    const int m2 = it % R2, r = it / R2;
+    float2 v[R1];
+#pragma unroll
+    for (int m1 = 0; m1 < R1; ++m1) v[m1] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int p = R2 * h + m2 + N * r;
+      float2 u = xi[p];
+      if (S) u = a.E ? cmul(u, cmul(S[p], a.E[p])) : cmul(S[p], u);
+      const float f = parity2(r + g.pad_off[0], R2 * h + m2 + n / 4) ? -a.deapf[p] : a.deapf[p];
+      u = make_float2(u.x * f, u.y * f);
+      v[R1 / 4 + h] = W ? cmul(W[p], u) : u;
+    }
+    dft<R1>(v, false);
+    float2* d = Wk + r * SM::RS + m2;
+    d[0] = v[0];
+#pragma unroll
+    for (int q = 1; q < R1; ++q) d[q * SM::S2] = twiddle(v[q], a.tw[q * R2 + m2], false);
+  }
+  __syncthreads();
+  for (int it = threadIdx.x; it < N * R1; it += T) {         // second pass: (row, k1)
+    const int k1 = it % R1, r = it / R1;
+    float2 v[R2];
+    const float2* s = Wk + r * SM::RS + k1 * SM::S2;
+#pragma unroll
+    for (int q = 0; q < R2; ++q) v[q] = s[q];
+    dft<R2>(v, false);
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) P[r * n + k1 + R1 * k2] = v[k2];
+  }
+  __syncthreads();
+  const uint32_t* ym = a.rows + l * R1;                      // columns some sample reaches
+  for (int it = threadIdx.x; it < n * R2; it += T) {         // x transform, first pass: (column, m2)
+    const int col = it % n, m2 = it / n;
+    if (!(ym[col % R1] >> (col / R1) & 1u)) continue;
+    float2 v[R1];
+#pragma unroll
+    for (int m1 = 0; m1 < R1; ++m1) v[m1] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int h = 0; h < H; ++h) v[R1 / 4 + h] = P[(R2 * h + m2) * n + col];
+    dft<R1>(v, false);
+    float2* d = Wk + m2 * n + col;
+    d[0] = v[0];
+#pragma unroll
+    for (int q = 1; q < R1; ++q) d[q * R2 * n] = twiddle(v[q], a.tw[q * R2 + m2], false);
+  }
+  __syncthreads();
+  float2* out = grids + (uint64_t)b * n * n;
+  for (int it = threadIdx.x; it < n * R1; it += T) {         // second pass: (column, k1)
+    const int col = it % n, k1 = it / n;
+    if (!(ym[col % R1] >> (col / R1) & 1u)) continue;
+    const uint32_t sup = xmask[((uint64_t)l * (n / 8) + col / 8) * R1 + k1];
+    float2 u[R2];
+    const float2* s = Wk + k1 * R2 * n + col;
+#pragma unroll
+    for (int q = 0; q < R2; ++q) u[q] = s[q * n];
+    dft<R2>(u, false);
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2)
+      if (sup >> k2 & 1u) out[(k1 + R1 * k2) * n + col] = u[k2];
+  }
+}
+
+template <int R1, int R2>
+__global__ void __launch_bounds__((GridGeo<R1, R2>::T)) k_fft2_inv_grid(NufftGeom g, FftRows a,
+                                                                       const uint32_t* __restrict__ xmask,
+                                                                       float2* grids, int clear, int accumulate,
+                                                                       float2* __restrict__ out) {
+  pdl_wait();
+  using GG = GridGeo<R1, R2>;
+  using SM = RowSm<R2, R1>;
+  constexpr int n = GG::n, N = GG::N, T = GG::T, H = R1 / 2;
+  extern __shared__ float2 sh[];
+  float2* Q = sh;                 // [cropped row][n]
+  float2* Wk = sh + GG::held;
+  const int b = blockIdx.x, c = b / a.L, l = b - c * a.L, cg = a.c0 + c;
+  const int img = a.cgroup > 0 ? cg / a.cgroup : 0;
+  const uint32_t* ym = a.rows + l * R1;
+  const float2* tw = a.tw + n;    // transposed: [k1 < R2][m2 < R1]
+  float2* in = grids + (uint64_t)b * n * n;
+  for (int it = threadIdx.x; it < n * R1; it += T) {         // x transform, first pass: (column, m2)
+    const int col = it % n, m2 = it / n;
+    if (!(ym[col % R1] >> (col / R1) & 1u)) continue;
+    const uint32_t sup = xmask[((uint64_t)l * (n / 8) + col / 8) * R1 + m2];
+    float2 v[R2];
+#pragma unroll
+    for (int m1 = 0; m1 < R2; ++m1) v[m1] = sup >> m1 & 1u ? in[(R1 * m1 + m2) * n + col] : make_float2(0.f, 0.f);
+    dft<R2>(v, true);
+    float2* d = Wk + m2 * n + col;
+    d[0] = v[0];
+#pragma unroll
+    for (int q = 1; q < R2; ++q) d[q * R1 * n] = twiddle(v[q], tw[q * R1 + m2], true);
+    if (clear) {
+#pragma unroll
+      for (int m1 = 0; m1 < R2; ++m1)
+        if (sup >> m1 & 1u) in[(R1 * m1 + m2) * n + col] = make_float2(0.f, 0.f);
+    }
+  }
+  __syncthreads();
+  for (int it = threadIdx.x; it < n * R2; it += T) {         // second pass: (column, k1 < R2)
+    const int col = it % n, k1 = it / n;
+    if (!(ym[col % R1] >> (col / R1) & 1u)) continue;
+    float2 u[R1];
+    const float2* s = Wk + k1 * R1 * n + col;
+#pragma unroll
+    for (int q = 0; q < R1; ++q) u[q] = s[q * n];
+    dft<R1>(u, true);
+#pragma unroll
+    for (int h = 0; h < H; ++h) Q[(k1 + R2 * h) * n + col] = u[R1 / 4 + h];
+  }
+  __syncthreads();
+  for (int it = threadIdx.x; it < N * R1; it += T) {         // y transform, first pass: (row, m2)
+    const int m2 = it % R1, r = it / R1;
+    const uint32_t sup = ym[m2];
+    float2 v[R2];
+#pragma unroll
+    for (int m1 = 0; m1 < R2; ++m1) v[m1] = sup >> m1 & 1u ? Q[r * n + R1 * m1 + m2] : make_float2(0.f, 0.f);
+    dft<R2>(v, true);
+    float2* d = Wk + r * SM::RS + m2;
+    d[0] = v[0];
+#pragma unroll
+    for (int q = 1; q < R2; ++q) d[q * SM::S2] = twiddle(v[q], tw[q * R1 + m2], true);
+  }
+  __syncthreads();
+  const float2* S = a.S ? a.S + (uint64_t)cg * N * N : nullptr;
+  const float2* W = a.W ? a.W + (uint64_t)img * a.phase_stride + (uint64_t)l * N * N : nullptr;
+  // the grid's image: to x (split 1), to memory, or into shared memory, where the
+  // cluster of the image's grids adds them in rank order
+  const bool cluster = a.split > 1 && a.cluster;
+  float2* o = cluster ? Q : a.split == 1 ? out + (uint64_t)img * a.image_stride : out + (uint64_t)b * N * N;
+  const bool add = a.split == 1 && accumulate;
+  for (int it = threadIdx.x; it < N * R2; it += T) {         // second pass: (row, k1 < R2)
+    const int k1 = it % R2, r = it / R2;
+    float2 u[R1];
+    const float2* s = Wk + r * SM::RS + k1 * SM::S2;
+#pragma unroll
+    for (int q = 0; q < R1; ++q) u[q] = s[q];
+    dft<R1>(u, true);
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int p = k1 + R2 * h + N * r;
+      float2 v = u[R1 / 4 + h];
+      if (W) v = cmul(v, W[p]);
+      if (S) v = a.E ? cmul(cmul(cconj(S[p]), cconj(a.E[p])), v) : cmul(v, cconj(S[p]));
+      const float f = parity2(r + g.crop_off[0], R2 * h + k1 + n / 4) ? -a.deapf[p] : a.deapf[p];
+      v = make_float2(v.x * f, v.y * f);
+      o[p] = add ? cadd(o[p], v) : v;
+    }
+  }
+  if (!cluster) return;
+  // every thread of every block of the cluster reaches both barriers
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  float2* xi = out + (uint64_t)img * a.image_stride;
+  for (int p = (int)cl.block_rank() * T + threadIdx.x; p < N * N; p += a.split * T) {
+    float2 v = *cl.map_shared_rank(Q + p, 0);
+    for (int q = 1; q < a.split; ++q) v = cadd(v, *cl.map_shared_rank(Q + p, q));
+    xi[p] = accumulate ? cadd(xi[p], v) : v;
+  }
+  cl.sync();   // no block leaves while another reads its shared memory
 }
 
 template <typename K>
@@ -415,13 +650,35 @@ pg_status rows_fwd(const NufftGeom& g, const FftRows& a, const float2* x, float2
   return PG_OK;
 }
 
+// Launch in clusters of `size` blocks along x, after the previous kernel (pdl_wait).
+template <typename Kern, typename... Args>
+pg_status launch_cluster(Kern kern, unsigned grid, int block, size_t smem, int size, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)size;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = size > 1 ? 2 : 1;
+  PG_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+  count_launch();
+  return PG_OK;
+}
+
 template <int R1, int R2>
 pg_status rows_inv(const NufftGeom& g, const FftRows& a, int nimages, const float2* Q, int accumulate, float2* out,
                    cudaStream_t s) {
   using RG = RowGeo<R1, R2>;
-  PG_LAUNCH_PDL((k_fft_inv_rows<R1, R2>), (unsigned)(nimages * a.split) * ceil_div((uint64_t)g.Nx * g.Nz, RG::RB),
-                RG::T, 0, s, g, a, nimages, Q, accumulate, out);
-  return PG_OK;
+  return launch_cluster(k_fft_inv_rows<R1, R2>,
+                        (unsigned)(nimages * a.split) * ceil_div((uint64_t)g.Nx * g.Nz, RG::RB), RG::T, 0,
+                        a.cluster ? a.split : 1, s,
+                        g, a, nimages, Q, accumulate, out);
 }
 
 template <int R1, int R2>
@@ -452,12 +709,37 @@ pg_status cols_inv(const FftLines& a, uint64_t nsets, float2* in, int clear, flo
   return PG_OK;
 }
 
+template <int R1, int R2>
+pg_status grid_fwd(const NufftGeom& g, const FftRows& a, const uint32_t* xmask, const float2* x, float2* grids,
+                   cudaStream_t s) {
+  using GG = GridGeo<R1, R2>;
+  PG_TRY(allow_smem(k_fft2_fwd_grid<R1, R2>, GG::smem));
+  PG_LAUNCH_PDL((k_fft2_fwd_grid<R1, R2>), (unsigned)(a.C * a.L), GG::T, GG::smem, s, g, a, xmask, x, grids);
+  return PG_OK;
+}
+
+template <int R1, int R2>
+pg_status grid_inv(const NufftGeom& g, const FftRows& a, const uint32_t* xmask, float2* grids, int clear,
+                   int accumulate, float2* out, cudaStream_t s) {
+  using GG = GridGeo<R1, R2>;
+  PG_TRY(allow_smem(k_fft2_inv_grid<R1, R2>, GG::smem));
+  return launch_cluster(k_fft2_inv_grid<R1, R2>, (unsigned)(a.C * a.L), GG::T, GG::smem, a.cluster ? a.split : 1, s, g, a,
+                        xmask, grids, clear, accumulate, out);
+}
+
 }  // namespace fftk
 
 template <int R1, int R2>
 const FftOps* fft_ops() {
-  static const FftOps ops{R1 * R2, fftk::rows_fwd<R1, R2>, fftk::cols_fwd<R1, R2>, fftk::cols_inv<R1, R2>,
-                          fftk::rows_inv<R1, R2>, fftk::RowGeo<R1, R2>::RB};
+  static const FftOps ops = [] {
+    FftOps o{R1 * R2, fftk::rows_fwd<R1, R2>, fftk::cols_fwd<R1, R2>, fftk::cols_inv<R1, R2>,
+             fftk::rows_inv<R1, R2>, fftk::RowGeo<R1, R2>::RB, fftk::RowGeo<R1, R2>::MINB, nullptr, nullptr};
+    if constexpr (R1 * R2 <= 64) {
+      o.grid_fwd = fftk::grid_fwd<R1, R2>;
+      o.grid_inv = fftk::grid_inv<R1, R2>;
+    }
+    return o;
+  }();
   return &ops;
 }
 

@@ -62,26 +62,26 @@ const FftOps* ops_for(int n) {
   return nullptr;
 }
 
-// x[img][p] (+)= the image's `split` partial images: 8 lanes per pixel, lane
-// k takes partials k, k+8, ..., added by a fixed xor butterfly.  An image whose
-// coils began in an earlier batch (img * cgroup < c0) is added to.
-__global__ void k_sum_images(uint64_t N, int split, const float2* __restrict__ part, int img0, uint64_t image_stride,
+// x[img][p] (+)= its `ng` partial images: 8 lanes per pixel, lane k takes images
+// k, k+8, ..., added by a fixed xor butterfly.  An image whose coils began in an
+// earlier batch (img * cgroup < c0) is added to.
+__global__ void k_sum_images(uint64_t N, int ng, const float2* __restrict__ images, int img0, uint64_t image_stride,
                              int accumulate, int cgroup, int c0, float2* __restrict__ x) {
   pdl_wait();
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int k = (int)(t & 7);
   const uint64_t p = t >> 3;
-  const int img = img0 + blockIdx.y;
-  part += (uint64_t)blockIdx.y * split * N;
+  images += (uint64_t)blockIdx.y * ng * N;
   float2 acc = make_float2(0.f, 0.f);
   if (p < N)
-    for (int b = k; b < split; b += 8) acc = cadd(acc, part[(uint64_t)b * N + p]);
+    for (int b = k; b < ng; b += 8) acc = cadd(acc, images[(uint64_t)b * N + p]);
 #pragma unroll
   for (int o = 4; o >= 1; o >>= 1) {
     acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
     acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
   }
   if (p < N && k == 0) {
+    const int img = img0 + blockIdx.y;
     float2* o = x + (uint64_t)img * image_stride + p;
     *o = accumulate || (cgroup > 0 && img * cgroup < c0) ? cadd(*o, acc) : acc;
   }
@@ -195,9 +195,21 @@ pg_status fftpass_support(const NufftGeom& g, uint64_t M, int L, int K, const ui
   return PG_OK;
 }
 
+// Small 2-D grids run both passes of a grid in one block while the batch is at
+// most one wave.
+static bool one_block_per_grid(const NufftGeom& g, const FftBatch& b, const FftOps* op) {
+  return g.dim == 2 && op->grid_fwd && b.C * b.L <= sm_count();
+}
+// The adjoint then writes one image per grid, so every image of the batch has
+// to have all of its coils in it.
+static bool one_image_per_grid(const NufftGeom& g, const FftBatch& b, const FftOps* op) {
+  return one_block_per_grid(g, b, op) && (b.cgroup == 0 || (b.c0 % b.cgroup == 0 && b.C % b.cgroup == 0));
+}
+
 static FftRows rows_args(const FftBatch& b, const FftSupport& sup, const float2* W, const float* deapf,
-                         const float2* tw, int split) {
-  return FftRows{b.L, b.C, b.c0, b.cgroup, b.image_stride, b.phase_stride, b.S, b.E, W, deapf, sup.ymask.p, tw, split};
+                         const float2* tw, int split, bool cluster = false) {
+  return FftRows{b.L, b.C, b.c0, b.cgroup, b.image_stride, b.phase_stride, b.S, b.E, W, deapf, sup.ymask.p, tw, split,
+                 cluster ? 1 : 0};
 }
 
 pg_status fftpass_forward(const NufftGeom& g, const FftBatch& b, const FftSupport& sup, const float2* x,
@@ -206,6 +218,8 @@ pg_status fftpass_forward(const NufftGeom& g, const FftBatch& b, const FftSuppor
   const int B = b.C * b.L;
   if (B > kMaxGridY) return set_error(PG_INVALID_ARG, "fft passes: batch of %d grids", B);
   const FftOps* op = ops_for(g.Gx);
+  if (one_block_per_grid(g, b, op))
+    return op->grid_fwd(g, rows_args(b, sup, Wo, deapf, tw, 1), sup.xmask.p, x, grids, s);
   const uint64_t plane = (uint64_t)g.Gx * g.Gy, rows = (uint64_t)g.Nx * g.Gy;
   const int row_blocks = (int)ceil_div((uint64_t)g.Nx * g.Nz, op->rows_per_block);
   const int split = std::min(b.L, std::max(1, wanted_blocks() / std::max(1, row_blocks * b.C) + 1));
@@ -229,39 +243,75 @@ pg_status fftpass_clear(const NufftGeom& g, const FftBatch& b, const FftSupport&
   return PG_OK;
 }
 
-int fftpass_partials(const NufftGeom& g, const FftBatch& b, int nimages) {
-  const FftOps* op = ops_for(g.Gx);
-  const int row_blocks = (int)ceil_div((uint64_t)g.Nx * g.Nz, op->rows_per_block);
-  const int per_image = std::max(1, b.C / std::max(1, nimages)) * b.L;
-  if (row_blocks * nimages >= wanted_blocks()) return 1;
-  return std::min(per_image, wanted_blocks() / std::max(1, row_blocks * nimages) + 1);
+static int batch_images(const FftBatch& b) {
+  return b.cgroup > 0 ? (b.c0 + b.C - 1) / b.cgroup - b.c0 / b.cgroup + 1 : 1;
+}
+
+// How the grids of an image are shared out and added in the last inverse pass:
+// one block (split 1), a cluster of `split` blocks, or images in memory.  A
+// cluster saves the images' way through memory and a launch (64^2 x 32, 4 shots, TV
+// solve 5.34 -> 5.02 ms); where 8 blocks per group of lines leave SMs idle, more
+// shares with images in memory win (208^2, 12 coils, L = 10, pair: clusters of 8 378
+// us, 11 shares 295 us).
+struct InverseSplit {
+  int split;
+  bool cluster;
+};
+static InverseSplit inverse_split(const NufftGeom& g, const FftBatch& b, const FftOps* op) {
+  const int nimages = batch_images(b);
+  if (one_image_per_grid(g, b, op)) {
+    const int grids = b.C / nimages * b.L;
+    return {grids, grids <= 8 && (grids & (grids - 1)) == 0};
+  }
+  const int blocks = std::max(1, (int)ceil_div((uint64_t)g.Nx * g.Nz, op->rows_per_block) * nimages);
+  const int per_image = std::max(1, b.C / nimages) * b.L;
+  const int wave = op->row_blocks_per_sm * sm_count();
+  if (8 * blocks < wave && per_image > 8) return {std::min(per_image, std::max(8, wave / blocks)), false};
+  // the cluster size whose waves take the least time, a share's time being 1 / split
+  int split = 1;
+  double least = 1e30;
+  for (int n = 1; n <= std::min(8, per_image); n *= 2) {
+    const double t = (double)((blocks * n + wave - 1) / wave) / n;
+    if (t < 0.95 * least) { least = t; split = n; }
+  }
+  return {split, split > 1};
+}
+
+uint64_t fftpass_images(const NufftGeom& g, const FftBatch& b) {
+  const InverseSplit is = inverse_split(g, b, ops_for(g.Gx));
+  return is.split == 1 || is.cluster ? 0 : (uint64_t)is.split * batch_images(b) * g.nimg();
 }
 
 pg_status fftpass_adjoint(const NufftGeom& g, const FftBatch& b, const FftSupport& sup, float2* grids, int clear,
-                          const float2* WoH, const float* deapf, const float2* tw, float2* Q, float2* Rimg,
+                          const float2* WoH, const float* deapf, const float2* tw, float2* Q, float2* images,
                           int accumulate, float2* x, cudaStream_t s) {
   const int B = b.C * b.L;
   if (B > kMaxGridY) return set_error(PG_INVALID_ARG, "fft passes: batch of %d grids", B);
   const uint64_t plane = (uint64_t)g.Gx * g.Gy, rows = (uint64_t)g.Nx * g.Gy, N = g.nimg();
-  const int img0 = b.cgroup > 0 ? b.c0 / b.cgroup : 0;
-  const int nimages = b.cgroup > 0 ? (b.c0 + b.C - 1) / b.cgroup - img0 + 1 : 1;
-  const int split = fftpass_partials(g, b, nimages);
+  const int nimages = batch_images(b);
   const FftOps* op = ops_for(g.Gx);
-  FftLines lx{plane, rows, (uint64_t)g.Gy, b.L, g.Nz, sup.ylist.p, sup.ny, sup.xmask.p, g.Gy / 8, tw};
-  if (g.dim == 2) {
-    PG_TRY(op->cols_inv(lx, b.C, grids, clear, Q, s));
+  const InverseSplit is = inverse_split(g, b, op);
+  const bool kept = is.split > 1 && !is.cluster;   // images in memory, added by one more launch
+  const FftRows ra = rows_args(b, sup, WoH, deapf, tw, is.split, is.cluster);
+  if (one_image_per_grid(g, b, op)) {
+    PG_TRY(op->grid_inv(g, ra, sup.xmask.p, grids, clear, accumulate, kept ? images : x, s));
   } else {
-    // z lines keeping the Nz cropped slabs, then x lines per slab keeping Nx rows
-    float2* Q1 = Q + (uint64_t)B * g.Nz * rows;
-    const FftLines lz{g.ngrid(), (uint64_t)g.Nz * plane, plane, b.L, 1, sup.xylist.p, sup.nxy, nullptr, 0,
-                      tw + 2 * g.Gx};
-    PG_TRY(ops_for(g.Gz)->cols_inv(lz, b.C, grids, clear, Q1, s));
-    PG_TRY(op->cols_inv(lx, (uint64_t)b.C * g.Nz, Q1, 0, Q, s));
+    FftLines lx{plane, rows, (uint64_t)g.Gy, b.L, g.Nz, sup.ylist.p, sup.ny, sup.xmask.p, g.Gy / 8, tw};
+    if (g.dim == 2) {
+      PG_TRY(op->cols_inv(lx, b.C, grids, clear, Q, s));
+    } else {
+      // z lines keeping the Nz cropped slabs, then x lines per slab keeping Nx rows
+      float2* Q1 = Q + (uint64_t)B * g.Nz * rows;
+      const FftLines lz{g.ngrid(), (uint64_t)g.Nz * plane, plane, b.L, 1, sup.xylist.p, sup.nxy, nullptr, 0,
+                        tw + 2 * g.Gx};
+      PG_TRY(ops_for(g.Gz)->cols_inv(lz, b.C, grids, clear, Q1, s));
+      PG_TRY(op->cols_inv(lx, (uint64_t)b.C * g.Nz, Q1, 0, Q, s));
+    }
+    PG_TRY(op->rows_inv(g, ra, nimages, Q, accumulate, kept ? images : x, s));
   }
-  PG_TRY(op->rows_inv(g, rows_args(b, sup, WoH, deapf, tw, split), nimages, Q, accumulate, split == 1 ? x : Rimg, s));
-  if (split == 1) return PG_OK;
-  PG_LAUNCH_PDL(k_sum_images, dim3(ceil_div(N * 8, 256), (unsigned)nimages), 256, 0, s, N, split, Rimg, img0,
-                b.image_stride, accumulate, b.cgroup, b.c0, x);
+  if (!kept) return PG_OK;
+  PG_LAUNCH_PDL(k_sum_images, dim3(ceil_div(N * 8, 256), (unsigned)nimages), 256, 0, s, N, is.split, images,
+                b.cgroup > 0 ? b.c0 / b.cgroup : 0, b.image_stride, accumulate, b.cgroup, b.c0, x);
   return PG_OK;
 }
 

@@ -33,14 +33,14 @@ pg_status fftpass_forward(const NufftGeom& g, const FftBatch& b, const FftSuppor
                           cudaStream_t s);
 // Zeroes the supported cells of the batch's 3-D grids.
 pg_status fftpass_clear(const NufftGeom& g, const FftBatch& b, const FftSupport& sup, float2* grids, cudaStream_t s);
-// Partial images per image that fftpass_adjoint writes to Rimg (1: none).
-int fftpass_partials(const NufftGeom& g, const FftBatch& b, int nimages);
+// Elements of the grids' images that fftpass_adjoint keeps in memory (0: none).
+uint64_t fftpass_images(const NufftGeom& g, const FftBatch& b);
 // grids: C * L grids in (after the spread), read in their supported cells;
 // with clear set the first pass zeroes each of them after reading it.
-// Q: fftpass_scratch elements; Rimg: fftpass_partials images per image;
+// Q: fftpass_scratch elements; images: fftpass_images elements;
 // x (+)= the images' sums in a fixed order.
 pg_status fftpass_adjoint(const NufftGeom& g, const FftBatch& b, const FftSupport& sup, float2* grids, int clear,
-                          const float2* WoH, const float* deapf, const float2* tw, float2* Q, float2* Rimg,
+                          const float2* WoH, const float* deapf, const float2* tw, float2* Q, float2* images,
                           int accumulate, float2* x, cudaStream_t s);
 
 }  // namespace pg

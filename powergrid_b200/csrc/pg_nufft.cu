@@ -2020,9 +2020,8 @@ pg_status nufft_adjoint(NufftPlan* p, const NufftBatch& b, const float2* y, floa
     if (p->own_fft) {
       PG_TRY(grow(p->work->fin, fftpass_scratch(g, B), s));
       const FftBatch fb{nb, L, c0, b.S, b.E, b.cgroup, b.image_stride, b.phase_stride};
-      const int nimages = b.cgroup > 0 ? (c0 + nb - 1) / b.cgroup - c0 / b.cgroup + 1 : 1;
-      const int parts = fftpass_partials(g, fb, nimages);
-      if (parts > 1) PG_TRY(grow(p->work->rimg, (uint64_t)parts * nimages * g.nimg(), s));
+      const uint64_t images = fftpass_images(g, fb);
+      if (images) PG_TRY(grow(p->work->rimg, images, s));
       ProfScope ps("fft_adj", s);
       PG_TRY(fftpass_adjoint(g, fb, bin->sup, target, self_clear, b.WoH, p->deapf.p, p->tw2d.p, p->work->fin.p,
                              p->work->rimg.p, acc, x, s));
