@@ -222,6 +222,43 @@ __device__ __forceinline__ double block_part_sum(const double* part, int nb, int
   return res;
 }
 
+// Everything a solve from x = 0 starts with, in one pass over y: the solver's
+// copy of y, Ax = A 0 = 0, the residual r = W (.) y, x = ddir = 0, sum W |y|^2
+// (norm_grad denominator, solve_pwls_pcg.hpp:42-46) and, in the last block, the
+// scalars and flags.  As a copy, three clears and three kernels these took 25 us
+// of a 3-step solve of 128 x 128, L = 8, 4 coils (359 us).
+__global__ void k_start(uint64_t ni, uint64_t nd, const float2* __restrict__ yin, const float* __restrict__ W,
+                        float2* __restrict__ ybuf, float2* __restrict__ Ax, float2* __restrict__ r,
+                        float2* __restrict__ x, float2* __restrict__ ddir, double* part, int nb, unsigned* counter,
+                        int pstride, double* sc, uint32_t* fl) {
+  {
+    const uint64_t oi = (uint64_t)blockIdx.y * ni, od = (uint64_t)blockIdx.y * nd;
+    x += oi; ddir += oi;
+    yin += od; W += od; ybuf += od; Ax += od; r += od;
+    part += (size_t)blockIdx.y * pstride; counter += blockIdx.y;
+    sc += (size_t)blockIdx.y * S_NSCAL; fl += (size_t)blockIdx.y * F_NFLAG;
+  }
+  const float2 zero = make_float2(0.f, 0.f);
+  const uint64_t n = ni > nd ? ni : nd;
+  double a = 0.0;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    if (i < nd) {
+      const float2 v = yin[i];
+      const float w = W[i];
+      ybuf[i] = v;
+      Ax[i] = zero;
+      r[i] = make_float2(w * v.x, w * v.y);
+      a += (double)w * ((double)v.x * v.x + (double)v.y * v.y);
+    }
+    if (i < ni) x[i] = ddir[i] = zero;
+  }
+  block_store2(a, 0.0, part, nb);
+  if (!last_block(counter)) return;
+  const double ywy = block_part_sum(part, nb, 0);
+  if (threadIdx.x < S_NSCAL) sc[threadIdx.x] = threadIdx.x == S_YWY ? ywy : 0.0;
+  if (threadIdx.x < F_NFLAG) fl[threadIdx.x] = 0;
+}
+
 // r = W (.) (y - Ax): the residual before the first iteration.
 __global__ void k_residual(uint64_t n, const float2* __restrict__ y, const float2* __restrict__ Ax,
                            const float* __restrict__ W, float2* __restrict__ r) {
@@ -973,17 +1010,19 @@ pg_status pcg_solve_device(pg_op_s* A, const float2* x0, const float* W, const f
   }
   Solver& S = cache->S;
   // inputs into the buffers the graph reads
-  PG_CUDA(cudaMemcpyAsync(cache->ybuf.p, y, nd * sizeof(float2), cudaMemcpyDeviceToDevice, s));
   if (W) PG_CUDA(cudaMemcpyAsync(cache->wbuf.p, W, nd * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  if (x0) PG_CUDA(cudaMemcpyAsync(S.x.p, x0, ni * sizeof(float2), cudaMemcpyDeviceToDevice, s));
-  else PG_CUDA(cudaMemsetAsync(S.x.p, 0, ni * sizeof(float2), s));
+  if (!x0) {
+    // The start is zero and so is Ax = A * 0 (:55), exactly: the operators are
+    // linear and their factors finite (the deapodization's NaNs are stored as 0).
+    const int nb = red_blocks(std::max(S.nd, S.ni));
+    PG_LAUNCH(k_start, dim3((unsigned)nb, (unsigned)S.nseg), kRed, 0, s, S.ni, S.nd, y, S.W, cache->ybuf.p, S.Ax.p,
+              S.r.p, S.x.p, S.ddir.p, S.part.p, nb, S.counter.p, S.pstride, S.sc.p, S.fl.p);
+    return pcg_iterate(A, cache, niter, xout, iters_dev, s, cancel);
+  }
+  PG_CUDA(cudaMemcpyAsync(cache->ybuf.p, y, nd * sizeof(float2), cudaMemcpyDeviceToDevice, s));
+  PG_CUDA(cudaMemcpyAsync(S.x.p, x0, ni * sizeof(float2), cudaMemcpyDeviceToDevice, s));
   PG_CUDA(cudaMemsetAsync(S.ddir.p, 0, ni * sizeof(float2), s));
-  // Ax = A * xInitial (:55).  Without x0 the start is zero and so is A * 0,
-  // exactly (the operators are linear and their factors finite: the
-  // deapodization's NaNs are stored as 0), so Ax is cleared instead.
-  pg_status st = PG_OK;
-  if (x0) st = A->forward(S.x.p, S.Ax.p, s);
-  else PG_CUDA(cudaMemsetAsync(S.Ax.p, 0, nd * sizeof(float2), s));
+  const pg_status st = A->forward(S.x.p, S.Ax.p, s);   // Ax = A * xInitial (:55)
   if (st != PG_OK) { A->pcg_cache.reset(); return st; }
   PG_LAUNCH(k_ywy, dim3((unsigned)S.nbd, (unsigned)S.nseg), kRed, 0, s, S.nd, S.y, S.W, S.part.p, S.nbd, S.pstride);
   PG_LAUNCH(k_scalar_init, (unsigned)S.nseg, 32, 0, s, S.part.p, S.nbd, S.pstride, S.sc.p, S.fl.p);
