@@ -297,9 +297,10 @@ struct TileGeo {
 // coil chunk) pairs, subproblems largest first.  Each block takes the next
 // item until none is left; the block that finds the queue empty last resets
 // it for the next launch.  Returns the item, or -1.
-__device__ __forceinline__ int next_item(unsigned* q, int nitems) {
+__device__ __forceinline__ int next_item(unsigned* q, int nitems, bool first) {
   __shared__ int item;
   __syncthreads();   // the previous item's shared memory is no longer in use
+  if (nitems <= (int)gridDim.x) return first ? (int)blockIdx.x : -1;   // at most one item per block: no queue
   if (threadIdx.x == 0) {
     int it = (int)atomicAdd(&q[0], 1u);
     if (it >= nitems) {
@@ -581,7 +582,9 @@ __global__ void __launch_bounds__(256) k_spread(NufftGeom g, TileShape t, const 
     for (int q = threadIdx.x; q < (np * 2 * CELLS) / 4; q += blockDim.x) z[q] = make_int4(0, 0, 0, 0);
   }
   if (threadIdx.x < 16) vmax[threadIdx.x] = 0u;
-  for (int item; (item = next_item(queue, nitems)) >= 0;) {
+  bool first_item = true;
+  for (int item; (item = next_item(queue, nitems, first_item)) >= 0;) {
+  first_item = false;
   const int4 sp = sub[item / nchunks];
   const int cfirst = c0 + (item % nchunks) * cc;
   const int tile = sp.x, first = sp.z, count = sp.w;
@@ -810,13 +813,19 @@ __global__ void __launch_bounds__(256, spread2d_min_blocks(CC * KK))
   float2* sv2 = reinterpret_cast<float2*>(sv);
   uint32_t* sst = reinterpret_cast<uint32_t*>(sv + (size_t)smax * NP2);
   for (int q = tid; q < NP * 2 * CELLS / 4; q += blockDim.x) reinterpret_cast<int4*>(tile)[q] = make_int4(0, 0, 0, 0);
+  bool first_item = true;
   for (;;) {
     __syncthreads();                   // the previous item's shared memory is no longer in use
     if (tid == 0) {
-      int it = (int)atomicAdd(&queue[0], 1u);
-      if (it >= nitems) {
-        it = -1;
-        if (atomicAdd(&queue[1], 1u) == gridDim.x - 1) { queue[0] = 0u; queue[1] = 0u; }
+      int it;
+      if (nitems <= (int)gridDim.x) {    // one item per block: no queue
+        it = first_item ? (int)blockIdx.x : -1;
+      } else {
+        it = (int)atomicAdd(&queue[0], 1u);
+        if (it >= nitems) {
+          it = -1;
+          if (atomicAdd(&queue[1], 1u) == gridDim.x - 1) { queue[0] = 0u; queue[1] = 0u; }
+        }
       }
       s_item = it;
       vmax = 0u;
@@ -826,6 +835,7 @@ __global__ void __launch_bounds__(256, spread2d_min_blocks(CC * KK))
     __syncthreads();
     const int item = s_item;
     if (item < 0) break;
+    first_item = false;
     const int4 sp = sub[item / nchunks];
     const int cfirst = (item % nchunks) * CC;
     const int ncl = min(CC, nb - cfirst);
@@ -1006,11 +1016,12 @@ __global__ void __launch_bounds__(256, spread2d_min_blocks(CC * KK))
 // window starts two cells on, and six of the eight warps keep their registers.
 // Cells are summed by one warp in sample order: deterministic, and in plain
 // FP32 (no fixed-point scale).
-// What bounds it is latency and issue at three blocks per SM (57 % of the issue
-// slots); the form before this one (one warp per sample, two int32 shared atomics
+// What bounds it is issue (57 % of the slots) and latency at three blocks per SM; the form before this one (one warp per sample, two int32 shared atomics
 // per cell, 32 per sample and plane) waited for the atomics.  Operator pairs on
 // one B200: 96^2 x 16, 8 coils, L = 6 1.86 -> 1.61 ms; 128^2 x 64, 2 shots, 4 coils,
-// L = 12 4.36 -> 4.12 ms.  The adjoint's error against 64 bits went from 1.4e-6 (the
+// L = 12 4.36 -> 4.12 ms; with the flush stepping through z (an item of 30 samples
+// spent a third of its instructions there) 1.055 -> 1.012 and 3.21 -> 3.14 ms, the
+// kernel 475 -> 430 and 438 -> 393 us.  The adjoint's error against 64 bits went from 1.4e-6 (the
 // fixed-point scale of a whole item) to 2e-7.
 // Tile layout [plane][15][15][16] float2, rows of odd x rotated by 8 cells: a
 // half-warp's two rows of 8 y taps fall into distinct banks.
@@ -1043,7 +1054,9 @@ __global__ void __launch_bounds__(256) k_spread3d(NufftGeom g, TileShape t, cons
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int dy = lane & 7, dx = lane >> 3;
   for (int q = tid; q < NP * CELLS / 2; q += 256) reinterpret_cast<float4*>(tile)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int item; (item = next_item(queue, nitems)) >= 0;) {
+  bool first_item = true;
+  for (int item; (item = next_item(queue, nitems, first_item)) >= 0;) {
+    first_item = false;
     const int4 sp = sub[item / nchunks];
     const int cfirst = (item % nchunks) * CC;
     const int ncl = min(CC, nb - cfirst);
@@ -1112,33 +1125,44 @@ __global__ void __launch_bounds__(256) k_spread3d(NufftGeom g, TileShape t, cons
         const float wyz = sw[i * 24 + 8 + dy] * wzv;
         const float w0 = sw[i * 24 + dx] * wyz, w1 = sw[i * 24 + dx + 4] * wyz;
         const float2 w0v = make_float2(w0, w0), w1v = make_float2(w1, w1);
+        if constexpr (NP == 2) {
+          const float4 v = reinterpret_cast<const float4*>(sv)[i];
+          a0[0] = __ffma2_rn(w0v, make_float2(v.x, v.y), a0[0]);
+          a1[0] = __ffma2_rn(w1v, make_float2(v.x, v.y), a1[0]);
+          a0[1] = __ffma2_rn(w0v, make_float2(v.z, v.w), a0[1]);
+          a1[1] = __ffma2_rn(w1v, make_float2(v.z, v.w), a1[1]);
+        } else {
 #pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const float2 v = sv[i * NP + p];
-          a0[p] = __ffma2_rn(w0v, v, a0[p]);
-          a1[p] = __ffma2_rn(w1v, v, a1[p]);
+          for (int p = 0; p < NP; ++p) {
+            const float2 v = sv[i * NP + p];
+            a0[p] = __ffma2_rn(w0v, v, a0[p]);
+            a1[p] = __ffma2_rn(w1v, v, a1[p]);
+          }
         }
       }
     }
     if (cur >= 0) put();
     __syncthreads();
-    // flush two cells (y, y + 1) per vector atomic, zeroing them for the next item
-    const uint64_t G = g.ngrid();
-    for (int q = tid; q < E * E * 8; q += 256) {
-      const int row = q >> 3, yy = (q & 7) * 2;
-      const int zz = row / E, xx = row - zz * E;
+    // flush two cells (y, y + 1) per vector atomic, zeroing them for the next
+    // item: a thread keeps its (x, pair) and steps through every second z plane
+    if (tid < E * 16) {
+      const int zz = tid / (E * 8), xx = tid % (E * 8) / 8, yy = (tid & 7) * 2;
       float4* p4 = reinterpret_cast<float4*>(tile + cell(zz, xx, yy));
-      const int gx = x0 + xx, gy = y0 + yy, gz = z0 + zz;
-      const bool inside = gx < g.Gx && gy < g.Gy && gz < g.Gz;
-      const uint64_t idx = (uint64_t)gy + (uint64_t)g.Gy * ((uint64_t)gx + (uint64_t)g.Gx * gz);
+      const bool inside = x0 + xx < g.Gx && y0 + yy < g.Gy;
+      const uint64_t G = g.ngrid(), plane = (uint64_t)g.Gx * g.Gy;
+      float2* o = grids + ((uint64_t)cfirst * L + lseg) * G + (uint64_t)(y0 + yy) +
+                  (uint64_t)g.Gy * ((uint64_t)(x0 + xx) + (uint64_t)g.Gx * (z0 + zz));
+      const int nz = min(E, g.Gz - z0);
+#pragma unroll 2
+      for (int z = zz; z < E; z += 2, p4 += E * 16, o += 2 * plane) {
 #pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        const int c = p / KK, j = p % KK;
-        const float4 v = p4[p * (CELLS / 2)];
-        if (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f) {
-          p4[p * (CELLS / 2)] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (inside && c < ncl)
-            atomicAdd(reinterpret_cast<float4*>(grids + ((uint64_t)(cfirst + c) * L + lseg + j) * G + idx), v);
+        for (int p = 0; p < NP; ++p) {
+          const int c = p / KK, j = p % KK;
+          const float4 v = p4[p * (CELLS / 2)];
+          if (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f) {
+            p4[p * (CELLS / 2)] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (inside && z < nz && c < ncl) atomicAdd(reinterpret_cast<float4*>(o + ((uint64_t)c * L + j) * G), v);
+          }
         }
       }
     }
