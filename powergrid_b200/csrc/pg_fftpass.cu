@@ -187,10 +187,17 @@ pg_status fftpass_support(const NufftGeom& g, uint64_t M, int L, int K, const ui
   }
   out->ny = (int)ylist.size();
   out->nxy = (int)xylist.size();
-  PG_TRY(out->ymask.upload(ymask.data(), ymask.size(), s));
-  PG_TRY(out->xmask.upload(xmask.data(), xmask.size(), s));
-  if (!ylist.empty()) PG_TRY(out->ylist.upload(ylist.data(), ylist.size(), s));
-  if (!xylist.empty()) PG_TRY(out->xylist.upload(xylist.data(), xylist.size(), s));
+  // one upload: [ymask][xmask][ylist][xylist]
+  std::vector<uint32_t> all(std::move(ymask));
+  const size_t ox = all.size(), oy = ox + xmask.size(), oxy = oy + ylist.size();
+  all.insert(all.end(), xmask.begin(), xmask.end());
+  all.insert(all.end(), ylist.begin(), ylist.end());
+  all.insert(all.end(), xylist.begin(), xylist.end());
+  PG_TRY(out->words.upload(all.data(), all.size(), s));
+  out->ymask = out->words.p;
+  out->xmask = out->words.p + ox;
+  out->ylist = out->words.p + oy;
+  out->xylist = out->words.p + oxy;
   PG_CUDA(cudaStreamSynchronize(s));   // the host lists are released on return
   return PG_OK;
 }
@@ -208,7 +215,7 @@ static bool one_image_per_grid(const NufftGeom& g, const FftBatch& b, const FftO
 
 static FftRows rows_args(const FftBatch& b, const FftSupport& sup, const float2* W, const float* deapf,
                          const float2* tw, int split, bool cluster = false) {
-  return FftRows{b.L, b.C, b.c0, b.cgroup, b.image_stride, b.phase_stride, b.S, b.E, W, deapf, sup.ymask.p, tw, split,
+  return FftRows{b.L, b.C, b.c0, b.cgroup, b.image_stride, b.phase_stride, b.S, b.E, W, deapf, sup.ymask, tw, split,
                  cluster ? 1 : 0};
 }
 
@@ -219,17 +226,17 @@ pg_status fftpass_forward(const NufftGeom& g, const FftBatch& b, const FftSuppor
   if (B > kMaxGridY) return set_error(PG_INVALID_ARG, "fft passes: batch of %d grids", B);
   const FftOps* op = ops_for(g.Gx);
   if (one_block_per_grid(g, b, op))
-    return op->grid_fwd(g, rows_args(b, sup, Wo, deapf, tw, 1), sup.xmask.p, x, grids, s);
+    return op->grid_fwd(g, rows_args(b, sup, Wo, deapf, tw, 1), sup.xmask, x, grids, s);
   const uint64_t plane = (uint64_t)g.Gx * g.Gy, rows = (uint64_t)g.Nx * g.Gy;
   const int row_blocks = (int)ceil_div((uint64_t)g.Nx * g.Nz, op->rows_per_block);
   const int split = std::min(b.L, std::max(1, wanted_blocks() / std::max(1, row_blocks * b.C) + 1));
   PG_TRY(op->rows_fwd(g, rows_args(b, sup, Wo, deapf, tw, split), x, P, s));
-  FftLines lx{rows, plane, (uint64_t)g.Gy, b.L, g.Nz, sup.ylist.p, sup.ny, sup.xmask.p, g.Gy / 8, tw};
+  FftLines lx{rows, plane, (uint64_t)g.Gy, b.L, g.Nz, sup.ylist, sup.ny, sup.xmask, g.Gy / 8, tw};
   if (g.dim == 2) return op->cols_fwd(lx, b.C, P, grids, s);
   // x lines per nonzero z-slab, then z lines over the supported (x, y) columns
   float2* P2 = P + (uint64_t)B * g.Nz * rows;
   PG_TRY(op->cols_fwd(lx, (uint64_t)b.C * g.Nz, P, P2, s));
-  const FftLines lz{(uint64_t)g.Nz * plane, g.ngrid(), plane, b.L, 1, sup.xylist.p, sup.nxy, nullptr, 0, tw + 2 * g.Gx};
+  const FftLines lz{(uint64_t)g.Nz * plane, g.ngrid(), plane, b.L, 1, sup.xylist, sup.nxy, nullptr, 0, tw + 2 * g.Gx};
   return ops_for(g.Gz)->cols_fwd(lz, b.C, P2, grids, s);
 }
 
@@ -238,7 +245,7 @@ pg_status fftpass_clear(const NufftGeom& g, const FftBatch& b, const FftSupport&
   const unsigned bx = ceil_div((uint64_t)sup.nxy * 4, 256);
   const int zsplit = std::max(1, std::min(g.Gz, kMaxGridY / std::max(1, b.C)));
   const int zs = std::min(zsplit, 16);
-  PG_LAUNCH_PDL(k_clear_groups, dim3(bx, (unsigned)(b.C * zs)), 256, 0, s, sup.xylist.p, sup.nxy, b.L,
+  PG_LAUNCH_PDL(k_clear_groups, dim3(bx, (unsigned)(b.C * zs)), 256, 0, s, sup.xylist, sup.nxy, b.L,
                 (uint64_t)g.Gx * g.Gy, g.Gz, zs, grids);
   return PG_OK;
 }
@@ -294,15 +301,15 @@ pg_status fftpass_adjoint(const NufftGeom& g, const FftBatch& b, const FftSuppor
   const bool kept = is.split > 1 && !is.cluster;   // images in memory, added by one more launch
   const FftRows ra = rows_args(b, sup, WoH, deapf, tw, is.split, is.cluster);
   if (one_image_per_grid(g, b, op)) {
-    PG_TRY(op->grid_inv(g, ra, sup.xmask.p, grids, clear, accumulate, kept ? images : x, s));
+    PG_TRY(op->grid_inv(g, ra, sup.xmask, grids, clear, accumulate, kept ? images : x, s));
   } else {
-    FftLines lx{plane, rows, (uint64_t)g.Gy, b.L, g.Nz, sup.ylist.p, sup.ny, sup.xmask.p, g.Gy / 8, tw};
+    FftLines lx{plane, rows, (uint64_t)g.Gy, b.L, g.Nz, sup.ylist, sup.ny, sup.xmask, g.Gy / 8, tw};
     if (g.dim == 2) {
       PG_TRY(op->cols_inv(lx, b.C, grids, clear, Q, s));
     } else {
       // z lines keeping the Nz cropped slabs, then x lines per slab keeping Nx rows
       float2* Q1 = Q + (uint64_t)B * g.Nz * rows;
-      const FftLines lz{g.ngrid(), (uint64_t)g.Nz * plane, plane, b.L, 1, sup.xylist.p, sup.nxy, nullptr, 0,
+      const FftLines lz{g.ngrid(), (uint64_t)g.Nz * plane, plane, b.L, 1, sup.xylist, sup.nxy, nullptr, 0,
                         tw + 2 * g.Gx};
       PG_TRY(ops_for(g.Gz)->cols_inv(lz, b.C, grids, clear, Q1, s));
       PG_TRY(op->cols_inv(lx, (uint64_t)b.C * g.Nz, Q1, 0, Q, s));

@@ -1397,12 +1397,13 @@ std::unique_ptr<Binning> binning_share(const Binning& b) {
   o->l0.borrow(b.l0);
   o->aa.borrow(b.aa);
   o->subprob.borrow(b.subprob);
-  o->sup.ylist.borrow(b.sup.ylist);
-  o->sup.xylist.borrow(b.sup.xylist);
-  o->sup.ymask.borrow(b.sup.ymask);
-  o->sup.xmask.borrow(b.sup.xmask);
-  o->sup.ny = b.sup.ny;
-  o->sup.nxy = b.sup.nxy;
+  if (b.sup) {
+    o->sup = std::make_shared<FftSupport>();
+    o->sup->words.borrow(b.sup->words);
+    o->sup->ylist = b.sup->ylist; o->sup->xylist = b.sup->xylist;
+    o->sup->ymask = b.sup->ymask; o->sup->xmask = b.sup->xmask;
+    o->sup->ny = b.sup->ny; o->sup->nxy = b.sup->nxy;
+  }
   return o;
 }
 
@@ -1412,7 +1413,7 @@ pg_status nufft_plain_binning(NufftPlan* p, cudaStream_t s) {
 }
 
 pg_status nufft_build_binning(NufftPlan* p, int L, int K, const int* l0_host, const float2* aa_host,
-                              std::unique_ptr<Binning>* out, cudaStream_t s) {
+                              std::unique_ptr<Binning>* out, cudaStream_t s, std::shared_ptr<FftSupport> sup) {
   const NufftGeom& g = p->g;
   const uint64_t M = p->M;
   auto b = std::make_unique<Binning>();
@@ -1435,8 +1436,13 @@ pg_status nufft_build_binning(NufftPlan* p, int L, int K, const int* l0_host, co
   PG_LAUNCH(k_prepare, ceil_div(M, 256), 256, 0, s, g, M, p->kx.p, p->ky.p, p->kz.p, p->lut.p, t,
             l0_host ? l0d.p : nullptr, st_o.p, wxy_o.p, g.dim == 3 ? wz_o.p : nullptr, key.p);
 
-  if (p->own_fft)
-    PG_TRY(fftpass_support(g, M, L, K, st_o.p, l0_host ? l0d.p : nullptr, &b->sup, s));
+  if (p->own_fft) {
+    b->sup = std::move(sup);
+    if (!b->sup) {
+      b->sup = std::make_shared<FftSupport>();
+      PG_TRY(fftpass_support(g, M, L, K, st_o.p, l0_host ? l0d.p : nullptr, b->sup.get(), s));
+    }
+  }
 
   // Stable counting sort by key on the device (bit-exact against a CPU one).
   DevBuf<uint32_t> starts_d;
@@ -1908,7 +1914,7 @@ pg_status nufft_forward(NufftPlan* p, const NufftBatch& b, const float2* x, floa
       PG_TRY(grow(p->work->fin, fftpass_scratch(g, B), s));
       ProfScope ps("fft_fwd", s);
       const FftBatch fb{nb, L, c0, b.S, b.E, b.cgroup, b.image_stride, b.phase_stride};
-      PG_TRY(fftpass_forward(g, fb, bin->sup, x, b.Wo, p->deapf.p, p->tw2d.p, p->work->fin.p, p->work->grids.p, s));
+      PG_TRY(fftpass_forward(g, fb, *bin->sup, x, b.Wo, p->deapf.p, p->tw2d.p, p->work->fin.p, p->work->grids.p, s));
     } else {
     cufftHandle h;
     PG_TRY(ensure_workspace(p, B, &h, s));
@@ -2002,7 +2008,7 @@ pg_status nufft_adjoint(NufftPlan* p, const NufftBatch& b, const float2* y, floa
       if (!self_clear) {
         // the own 3-D passes read only the supported cells
         ProfScope ps("prep", s);
-        if (p->own_fft) PG_TRY(fftpass_clear(g, FftBatch{nb, L}, bin->sup, target, s));
+        if (p->own_fft) PG_TRY(fftpass_clear(g, FftBatch{nb, L}, *bin->sup, target, s));
         else PG_CUDA(cudaMemsetAsync(target, 0, (size_t)B * G * sizeof(float2), s));
       }
       p->work->agrids_clean = false;
@@ -2047,7 +2053,7 @@ pg_status nufft_adjoint(NufftPlan* p, const NufftBatch& b, const float2* y, floa
       const uint64_t images = fftpass_images(g, fb);
       if (images) PG_TRY(grow(p->work->rimg, images, s));
       ProfScope ps("fft_adj", s);
-      PG_TRY(fftpass_adjoint(g, fb, bin->sup, target, self_clear, b.WoH, p->deapf.p, p->tw2d.p, p->work->fin.p,
+      PG_TRY(fftpass_adjoint(g, fb, *bin->sup, target, self_clear, b.WoH, p->deapf.p, p->tw2d.p, p->work->fin.p,
                              p->work->rimg.p, acc, x, s));
       if (self_clear) p->work->agrids_clean = true;   // the first inverse pass leaves the target zero
       continue;

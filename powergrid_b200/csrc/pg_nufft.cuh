@@ -47,11 +47,13 @@ struct NufftTune {
 // Grid cells that a segmentation's taps reach, in groups of 8 adjacent y
 // cells (pg_fftpass.cu).  The own FFT passes leave every other cell alone.
 struct FftSupport {
-  DevBuf<uint32_t> ylist;    // segment << 24 | y group, with a tap at any x (ny entries)
-  DevBuf<uint32_t> xylist;   // segment << 24 | x * (Gy / 8) + y group (3-D, nxy entries)
+  DevBuf<uint32_t> words;              // the four tables below
+  const uint32_t* ylist = nullptr;     // segment << 24 | y group, with a tap at any x (ny entries)
+  const uint32_t* xylist = nullptr;    // segment << 24 | x * (Gy / 8) + y group (3-D, nxy entries)
   // support words of a thread's grid rows r + R1 q, bit q: [segment][R1] along
   // y, [segment][y group][R1] along x
-  DevBuf<uint32_t> ymask, xmask;
+  const uint32_t* ymask = nullptr;
+  const uint32_t* xmask = nullptr;
   int ny = 0, nxy = 0;
 };
 
@@ -72,7 +74,7 @@ struct Binning {
   DevBuf<float2> aa;         // K per sample: interpolator values AA(m, l0..l0+K-1)
   DevBuf<int4> subprob;      // (tile index, l0, first sorted sample, count)
   DevBuf<uint32_t> keys;     // bin key per original sample
-  FftSupport sup;            // for the own FFT passes
+  std::shared_ptr<FftSupport> sup;   // for the own FFT passes; the same for every tile and bin size
   int nsub = 0;
   int submax = 0;            // most samples in one subproblem
   uint64_t nkeys = 0;
@@ -138,8 +140,10 @@ pg_status nufft_plan_create(std::unique_ptr<NufftPlan>* out, uint64_t M, float g
                             const float* kx, const float* ky, const float* kz, cudaStream_t s);
 // Binning for a segmentation: l0_host/aa_host (K per sample, original order)
 // or null for the unsegmented case.
+// sup: the support of an earlier binning of the same samples and windows, or null.
 pg_status nufft_build_binning(NufftPlan* p, int L, int K, const int* l0_host, const float2* aa_host,
-                              std::unique_ptr<Binning>* out, cudaStream_t s);
+                              std::unique_ptr<Binning>* out, cudaStream_t s,
+                              std::shared_ptr<FftSupport> sup = nullptr);
 pg_status nufft_plain_binning(NufftPlan* p, cudaStream_t s);
 // A plan that reads src's trajectory tables (src must outlive it) and has a
 // workspace of its own, so it can run concurrently with src on another stream.

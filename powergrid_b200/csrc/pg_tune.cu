@@ -90,7 +90,8 @@ pg_status nufft_autotune(NufftPlan* p, int L, int K, const int* l0_host, const f
       const bool rebin = (g.dim == 2 ? t.tile2d != p->tune.tile2d : t.tile3d != p->tune.tile3d) ||
                          (g.dim == 2 ? t.submax2d != p->tune.submax2d : t.submax3d != p->tune.submax3d);
       p->tune = t;
-      if (rebin || !*bin) return nufft_build_binning(p, L, K, l0_host, aa_host, bin, s);
+      if (rebin || !*bin)
+        return nufft_build_binning(p, L, K, l0_host, aa_host, bin, s, *bin ? (*bin)->sup : nullptr);
       return PG_OK;
     }
   }
@@ -117,6 +118,7 @@ pg_status nufft_autotune(NufftPlan* p, int L, int K, const int* l0_host, const f
   const std::vector<int> submaxes = {128, 256, 512};
   NufftTune best = base;
   std::unique_ptr<Binning> best_bin;
+  std::shared_ptr<FftSupport> sup = *bin ? (*bin)->sup : nullptr;
   float best_ms = 3e30f;
   for (int tile : tiles)
     for (int sm : submaxes) {
@@ -124,7 +126,8 @@ pg_status nufft_autotune(NufftPlan* p, int L, int K, const int* l0_host, const f
       if (g.dim == 2) { t.tile2d = tile; t.submax2d = sm; } else { t.tile3d = tile; t.submax3d = sm; }
       p->tune = t;
       std::unique_ptr<Binning> cand;
-      PG_TRY(nufft_build_binning(p, L, K, l0_host, aa_host, &cand, s));
+      PG_TRY(nufft_build_binning(p, L, K, l0_host, aa_host, &cand, s, sup));
+      sup = cand->sup;
       NufftBatch b;
       b.C = Ct;
       b.bin = cand.get();
