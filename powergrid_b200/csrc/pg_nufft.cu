@@ -431,11 +431,14 @@ __global__ void __launch_bounds__(128) k_gather(NufftGeom g, TileShape t, const 
 // (0.6 per cell).
 // Taps outside the clamped window weigh 0 and, where they lie outside the grid,
 // are not read.
+// One or two planes are held to 40 registers, six blocks per SM, for the loads'
+// latency.  With 48 and five blocks an operator pair at 96^2 x 16 took 1.01 ms and
+// one at 128^2 x 64 3.14 ms; with 40, 0.99 and 3.06 ms.
 // ---------------------------------------------------------------------------
 constexpr int kGatherRun = 64;    // samples per block: two passes of 32
 
 template <int CC, int KP>
-__global__ void __launch_bounds__(256) k_gather3d(NufftGeom g, uint64_t M, const uint2* __restrict__ start,
+__global__ void __launch_bounds__(256, CC * KP <= 2 ? 6 : 1) k_gather3d(NufftGeom g, uint64_t M, const uint2* __restrict__ start,
                                                   const float* __restrict__ wxy, const float* __restrict__ wz,
                                                   const uint32_t* __restrict__ perm, const int* __restrict__ l0,
                                                   const float2* __restrict__ aa, int K, int L,
@@ -1725,7 +1728,7 @@ static pg_status launch_gather_t(NufftPlan* p, const Binning* bin, const float2*
 
 // 3-D gather launch: CC coils x KP segments per pass, at most 8 planes (16
 // accumulator registers and 8 loads in flight per tap).  The tuner takes one
-// coil at the configurations' sizes: 48 registers, twice the warps of four coils.
+// coil at the configurations' sizes: 40 registers, more warps than four coils.
 template <int CC, int KP>
 static pg_status gather3d_launch_one(NufftPlan* p, const Binning* bin, const float2* aa, int nb, float2* y,
                                    uint64_t dstride, cudaStream_t s) {
