@@ -1071,7 +1071,11 @@ __global__ void __launch_bounds__(256) k_spread3d(NufftGeom g, TileShape t, cons
     for (int p = 0; p < NP; ++p) a0[p] = a1[p] = make_float2(0.f, 0.f);
     int cur = -1;                          // ox | oy << 8 | z << 16 of the cells in registers
     float2* c0 = tile;
+    // Every lane of the warp comes here (the loop's branches are uniform).  A cell
+    // of this window may have been stored by another lane at the window before:
+    // the barrier orders that store before the load below.
     auto put = [&]() {
+      __syncwarp();
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         float2* q = c0 + p * CELLS;

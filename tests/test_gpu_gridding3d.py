@@ -67,3 +67,25 @@ def test_gridding_3d_planes_vs_oracle(pg, oracle, L, interp, nc):
     So = oracle.sense(Ao, sm, M, N, nc)
     assert rel_l2(Sg * x, So.forward(x)) <= OP_TOL
     assert rel_l2(Sg / y, So.adjoint(y)) <= OP_TOL
+
+
+@pytest.mark.parametrize("L,nc", [(1, 1), (1, 4), (4, 3)])
+def test_spread_hands_cells_between_lanes(pg, oracle, L, nc):
+    """Windows that move by one cell from sample to sample, in every direction: each
+    cell of the tile passes between the lanes that add to it."""
+    from powergrid_b200 import synthetic as S
+    n, nz = 16, 8
+    c = (np.arange(-20, 20) / 10.0).astype(np.float32)      # 8 windows per axis, several samples in each
+    kx, ky = (a.ravel() for a in np.meshgrid(c, c, indexing="ij"))
+    kz = np.resize(np.float32([-0.6, -0.1, 0.3]), kx.size)
+    t = np.linspace(0, 8e-3, kx.size).astype(np.float32)
+    M, N = kx.size, n * n * nz
+    fm, sm = S.field_map(S.Rng(5), n, n, nz, 60.0), S.coil_maps(S.Rng(6), n, n, nz, nc)
+    A, Ao = pg.Gnufft(M, 2.0, n, n, nz, kx, ky, kz), oracle.gnufft(0, M, n, n, nz, kx, ky, kz)
+    if L > 1:
+        A, Ao = pg.TimeSegmentation(A, fm, t, M, N, L, 1, 1), oracle.timeseg(Ao, fm, t, M, N, L)
+    Sg, So = pg.SENSE(A, sm, M, N, nc), oracle.sense(Ao, sm, M, N, nc)
+    y = S.image(S.Rng(7), M * nc)
+    want = So.adjoint(y)
+    for _ in range(3):
+        assert rel_l2(Sg / y, want) <= OP_TOL
