@@ -114,6 +114,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
+// Waits for the matrix products committed to `bar`.  They have then read their
+// operands and written D: the fence orders this thread's next tcgen05.st (which
+// overwrites A) and tcgen05.ld (which takes D) after them.
+__device__ __forceinline__ bool product_wait(uint32_t bar, uint32_t parity) {
+  const bool done = mbar_wait(bar, parity);
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  return done;
+}
+
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }
@@ -261,7 +270,6 @@ __global__ void __launch_bounds__((Tc<NC>::TO), 1)
 
   // adds columns [0, V) at d to the sums
   auto take = [&](uint32_t d) {
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
     for (int h = 0; h < V / 16; ++h) {
       uint32_t r[16];
@@ -320,7 +328,7 @@ __global__ void __launch_bounds__((Tc<NC>::TO), 1)
         }
         if (h == 0 && pending) {
           // the previous step's product has read A and B and written D
-          if (ok) ok = mbar_wait(bar, parity);
+          if (ok) ok = product_wait(bar, parity);
           parity ^= 1;
           pending = false;
           if (ch % kDrain == 0) {
@@ -361,7 +369,7 @@ __global__ void __launch_bounds__((Tc<NC>::TO), 1)
     }
   }
   if (pending) {
-    if (ok) ok = mbar_wait(bar, parity);
+    if (ok) ok = product_wait(bar, parity);
     take(tD);
     take(tD + V);
     fold();

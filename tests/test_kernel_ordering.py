@@ -41,3 +41,18 @@ def test_spread3d_orders_a_cells_lanes(step):
     assert any(a[c] != b[c] for c in a.keys() & b.keys())
     body = _block(_source("pg_nufft.cu").split("void __launch_bounds__(256) k_spread3d(", 1)[1], "auto put = [&]()")
     assert re.match(r"\s*__syncwarp\(\);", body)
+
+
+def test_tensor_operand_is_rewritten_after_the_product_that_read_it():
+    """k_tc_dft overwrites A in tensor memory (tcgen05.st) once the matrix product that
+    read it is complete, and then takes D (tcgen05.ld).  Both need
+    tcgen05.fence::after_thread_sync behind the wait on the product's mbarrier, at every
+    step: the wait and the fence are one function, and nothing waits without it."""
+    src = _source("pg_gdft_tc.cu")
+    wait = _block(src, "bool product_wait(")
+    assert re.search(r"mbar_wait\(bar, parity\);\s*asm volatile\(\"tcgen05\.fence::after_thread_sync;", wait)
+    kernel = _block(src.split("k_tc_dft(", 1)[1], ") {")
+    assert "mbar_wait(" not in kernel and len(re.findall(r"= product_wait\(", kernel)) == 2
+    step = _block(kernel, "if (h == 0 && pending)")
+    assert step.index("product_wait(") < step.index("take(") and "tm_store16(" not in step
+    assert kernel.index("product_wait(") < kernel.index("tm_store16(tA")
