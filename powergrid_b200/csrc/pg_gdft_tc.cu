@@ -369,7 +369,10 @@ __global__ void __launch_bounds__((Tc<NC>::TO), 1)
     }
   }
   if (pending) {
-    if (ok) ok = product_wait(bar, parity);
+    // also where an earlier wait ran out: no product should be in flight when
+    // tensor memory is freed
+    const bool done = product_wait(bar, parity);
+    ok = ok && done;
     take(tD);
     take(tD + V);
     fold();
