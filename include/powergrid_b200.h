@@ -136,7 +136,8 @@ pg_status pg_op_forward(pg_op op, const float* x, float* y);
 pg_status pg_op_adjoint(pg_op op, const float* y, float* x);
 
 /* The same on DEVICE buffers, stream-ordered (stream may be NULL = the
- * library's default stream).  No host synchronisation. */
+ * library's default stream, a blocking one: it is ordered with the work of the
+ * legacy default stream, before and after).  No host synchronisation. */
 pg_status pg_op_forward_device(pg_op op, const void* x_dev, void* y_dev, void* stream);
 pg_status pg_op_adjoint_device(pg_op op, const void* y_dev, void* x_dev, void* stream);
 

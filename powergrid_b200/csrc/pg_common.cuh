@@ -23,6 +23,17 @@ pg_status set_error(pg_status s, const char* fmt, ...);
 void noalloc_forget_scratch();
 pg_status ensure_init();
 cudaStream_t default_stream();
+// The stream on which to capture a graph that will be launched on `on`.
+struct CaptureStream {
+  cudaStream_t s;
+  explicit CaptureStream(cudaStream_t on);
+  ~CaptureStream();
+  CaptureStream(const CaptureStream&) = delete;
+  CaptureStream& operator=(const CaptureStream&) = delete;
+
+ private:
+  cudaStream_t own = nullptr;
+};
 int sm_count();
 
 // Counts this library's kernel launches (reported by bench.py).

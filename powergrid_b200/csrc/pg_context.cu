@@ -39,6 +39,8 @@ bool g_inited = false;
 int g_device = 0;
 int g_sms = 148;
 cudaStream_t g_stream = nullptr;
+std::mutex g_capture_mu;
+std::vector<cudaStream_t> g_capture_free;   // non-blocking, for CaptureStream
 }  // namespace
 
 pg_status set_error(pg_status s, const char* fmt, ...) {
@@ -79,12 +81,39 @@ pg_status ensure_init() {
     }
     cudaGetLastError();
   }
-  PG_CUDA(cudaStreamCreateWithFlags(&g_stream, cudaStreamNonBlocking));
+  // A blocking stream: its work waits for what is already on the legacy default
+  // stream, and later work there waits for it.  Callers that name no stream (NULL)
+  // make and read their buffers on the legacy stream: PyTorch's default one.
+  PG_CUDA(cudaStreamCreateWithFlags(&g_stream, cudaStreamDefault));
+  cudaStream_t capture = nullptr;
+  PG_CUDA(cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking));
+  g_capture_free.push_back(capture);
   g_inited = true;
   return PG_OK;
 }
 
 cudaStream_t default_stream() { return g_stream; }
+
+// While a blocking stream is captured, any thread's work on the legacy stream
+// would be an implicit dependency on the capture, an error for both.  So the
+// default stream's graphs are captured on a non-blocking one and launched on it.
+// Those streams are kept, as many as captures ever ran at once: making and
+// destroying one took 100 us of a new operator's first 64 x 64 solve (0.35 ms).
+CaptureStream::CaptureStream(cudaStream_t on) : s(on) {
+  if (on != g_stream) return;
+  std::lock_guard<std::mutex> lk(g_capture_mu);
+  if (!g_capture_free.empty()) {
+    s = own = g_capture_free.back();
+    g_capture_free.pop_back();
+  } else if (cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) == cudaSuccess) {
+    s = own;
+  }
+}
+CaptureStream::~CaptureStream() {
+  if (!own) return;
+  std::lock_guard<std::mutex> lk(g_capture_mu);
+  g_capture_free.push_back(own);
+}
 int sm_count() { return g_sms; }
 
 namespace {
@@ -186,6 +215,11 @@ pg_status pg_shutdown(void) {
   cudaStreamSynchronize(pg::g_stream);
   cudaStreamDestroy(pg::g_stream);
   pg::g_stream = nullptr;
+  {
+    std::lock_guard<std::mutex> lc(pg::g_capture_mu);
+    for (cudaStream_t c : pg::g_capture_free) cudaStreamDestroy(c);
+    pg::g_capture_free.clear();
+  }
   pg::noalloc_forget_scratch();
   pg::g_inited = false;
   return PG_OK;

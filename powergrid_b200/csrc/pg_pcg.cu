@@ -1038,9 +1038,10 @@ void capture_chunk(PcgCache* cache, cudaStream_t s) {
   pg_status st = PG_OK;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-    for (int k = 0; k < kChunk && st == PG_OK; ++k) st = cache->S.iteration(s);
-    cudaError_t ce = cudaStreamEndCapture(s, &graph);
+  const CaptureStream cap(s);
+  if (cudaStreamBeginCapture(cap.s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+    for (int k = 0; k < kChunk && st == PG_OK; ++k) st = cache->S.iteration(cap.s);
+    cudaError_t ce = cudaStreamEndCapture(cap.s, &graph);
     if (st == PG_OK && ce == cudaSuccess) ce = cudaGraphInstantiate(&exec, graph, 0);
     if (st == PG_OK && ce == cudaSuccess) {
       cache->graph_chunk = graph;
@@ -1073,10 +1074,11 @@ pg_status pcg_iterate(pg_op_s* A, PcgCache* cache, uint64_t niter, float2* xout,
       for (int timed = 0; timed < (g_profile ? 2 : 1); ++timed) {
         const uint64_t before = g_launches.load();
         g_profile_suppress = timed == 0;
-        PG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        st = S.iteration(s);
+        const CaptureStream cap(s);
+        PG_CUDA(cudaStreamBeginCapture(cap.s, cudaStreamCaptureModeThreadLocal));
+        st = S.iteration(cap.s);
         cudaGraph_t graph = nullptr;
-        cudaError_t ce = cudaStreamEndCapture(s, &graph);
+        cudaError_t ce = cudaStreamEndCapture(cap.s, &graph);
         g_profile_suppress = false;
         // the capture pass counted launches that never ran
         cache->per_iter = g_launches.load() - before;
@@ -1488,10 +1490,11 @@ pg_status pcg_solve_lowrank(pg_op_s* A, const pg_penalty& Rh, uint64_t rank, con
     if (graphs_enabled() && niter > 1) {
       const uint64_t before = g_launches.load();
       g_profile_suppress = true;
-      PG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      st = c->iteration(A, s);
+      const CaptureStream cap(s);
+      PG_CUDA(cudaStreamBeginCapture(cap.s, cudaStreamCaptureModeThreadLocal));
+      st = c->iteration(A, cap.s);
       cudaGraph_t graph = nullptr;
-      cudaError_t ce = cudaStreamEndCapture(s, &graph);
+      cudaError_t ce = cudaStreamEndCapture(cap.s, &graph);
       g_profile_suppress = false;
       c->per_iter = g_launches.load() - before;
       g_launches.fetch_sub(c->per_iter);
