@@ -7,10 +7,10 @@
 // is formed in turns with FP64 products and reduced mod 1 in FP64, then one
 // FP32 __sincosf serves every coil of the pair.
 //
-// Two sets of kernels.  From kTensorCoils coils on, the sums over the pairs run
-// on the tensor cores (pg_gdft_tc.cu); below that, and for plans whose phases
-// its fixed-point form cannot hold, here: complex MACs in FP32 with a two-level
-// (per-tile, then running) sum.
+// Two sets of kernels.  The sums over the pairs run on the tensor cores
+// (pg_gdft_tc.cu) where these are the faster ones (use_tensor) and the plan's
+// phases fit their fixed-point form; elsewhere here: complex MACs in FP32 with a
+// two-level (per-tile, then running) sum.
 //
 // GdftR2 (ftCpuWithGrads.cpp:93-216) multiplies each pair by
 //   sinc(kx_i/Nx + Gx_j t_i) sinc(ky_i/Ny + Gy_j t_i) sinc(kz_i/Nz + Gz_j t_i),
@@ -347,26 +347,50 @@ static pg_status launch_adj(GdftPlan* p, int nsplit, uint64_t ichunk, const floa
 
 // Where the tensor cores' sums are the faster ones.  Their cost does not depend
 // on the number of coils up to 8 (then up to 16): at 64^2 x 32, 131072 samples,
-// 8 coils 20.7 ms against 34.5 ms; 47^2 x 8, 56544 samples, 13 coils with gradients
+// 8 coils 20.8 ms against 34.8 ms; 47^2 x 8, 56544 samples, 13 coils with gradients
 // 6.8 against 13.3 ms; 36^2 x 11, 2 x 11231 samples, 3 coils, both directions 0.95
-// against 1.14 ms.  With 1 or 2 coils the plain kernels have the fewer
+// against 1.16 ms.  With 1 or 2 coils the plain kernels have the fewer
 // instructions per pair.  Small sums do not make up for the packing launches and
 // the start of a CTA: 2304 voxels x 1636 samples, 6 coils, 4 shots, both
 // directions 418 against 397 us.
+//
+// Up to 8 coils it also depends on how the outputs fill the tensor kernel's CTAs:
+// 1024 outputs each, one CTA per SM, at most 64 splits of whole 128-input tiles.
+// (Few outputs: 1100 from 244033 inputs, 3 coils 757 us against 505 us.  Few inputs:
+// 83887 outputs from 400, 3 coils 116 against 75 us.)  So the tiles that the
+// busiest SM goes through on either side are compared, a tensor tile (1024
+// outputs) weighing as many plain ones (128 outputs) as fits 534 measurements of
+// both (2^25 to 2^28 pairs, 400 to 671089 outputs, 3, 5 and 8 coils, with and
+// without gradients): the kernel taken is at most 7 % behind the other one, 0.1-0.3 %
+// on average.  The pairs alone gave up to 92 % (400 outputs, 3 coils).  From 9 coils on the tensor cores won
+// everywhere (at worst 1.2 % behind: 83887 outputs from 400, 17 coils).
 constexpr int kTensorCoils = 3;
 constexpr uint64_t kTensorPairs = 1ull << 25;
 
-static bool use_tensor(const GdftPlan& p, int C) {
-  return p.turns_fit && C >= kTensorCoils && p.nk * p.ni >= kTensorPairs;
+// 128 x 128 tiles that the busiest SM of the plain kernels goes through.  An SM
+// needs about four resident blocks to be busy.
+static double plain_steps(uint64_t nout, uint64_t ninner) {
+  const uint64_t ns = (uint64_t)splits_for(nout, ninner), sms = (uint64_t)sm_count();
+  const uint64_t tiles = (ninner + kTile - 1) / kTile, chunk = (tiles + ns - 1) / ns;   // tiles per split
+  const uint64_t blocks = (nout + kTile - 1) / kTile * ((tiles + chunk - 1) / chunk);
+  const double per_sm = blocks > 8 * sms ? (double)blocks / (double)sms : (double)((blocks + sms - 1) / sms);
+  return std::max(4.0, per_sm) * std::min((double)chunk, (double)ninner / kTile);
+}
+
+static bool use_tensor(const GdftPlan& p, int C, uint64_t nout, uint64_t ninner) {
+  if (!p.turns_fit || C < kTensorCoils || p.nk * p.ni < kTensorPairs) return false;
+  if (C > 8) return true;
+  const double weight = p.kn.p ? 7.0 : C <= 4 ? 6.6 : 5.0;
+  return weight * (double)gdft_tc_split(nout, ninner, 8).steps <= plain_steps(nout, ninner);
 }
 
 static int pad_coils(int nc) { return nc <= 1 ? 1 : nc <= 2 ? 2 : nc <= 4 ? 4 : 8; }
 
 pg_status gdft_forward(GdftPlan* p, int C, const float2* S, const float2* x, float2* y, uint64_t dstride,
                        cudaStream_t s) {
-  if (use_tensor(*p, C)) {
+  if (use_tensor(*p, C, p->nk, p->ni)) {
     const GdftSide g{p->nk, p->ni, p->ks.p, p->vs.p, p->kn.p, p->gm.p, true};
-    const int ncp = gdft_tc_coils(C), ns = gdft_tc_splits(p->nk, p->ni, ncp);
+    const int ncp = gdft_tc_coils(C), ns = gdft_tc_split(p->nk, p->ni, ncp).splits;
     PG_TRY(grow(p->work->B, gdft_tc_operand(p->ni, ncp), s));
     PG_TRY(grow(p->work->part, (uint64_t)ns * ncp * p->nk, s));
     for (int c0 = 0; c0 < C; c0 += ncp) {
@@ -404,9 +428,9 @@ pg_status gdft_forward(GdftPlan* p, int C, const float2* S, const float2* x, flo
 
 pg_status gdft_adjoint(GdftPlan* p, int C, const float2* S, const float2* y, uint64_t dstride, float2* x,
                        cudaStream_t s) {
-  if (use_tensor(*p, C)) {
+  if (use_tensor(*p, C, p->ni, p->nk)) {
     const GdftSide g{p->ni, p->nk, p->vs.p, p->ks.p, p->gm.p, p->kn.p, false};
-    const int ncp = gdft_tc_coils(C), ns = gdft_tc_splits(p->ni, p->nk, ncp);
+    const int ncp = gdft_tc_coils(C), ns = gdft_tc_split(p->ni, p->nk, ncp).splits;
     PG_TRY(grow(p->work->B, gdft_tc_operand(p->nk, ncp), s));
     PG_TRY(grow(p->work->part, (uint64_t)ns * ncp * p->ni, s));
     for (int c0 = 0; c0 < C; c0 += ncp) {

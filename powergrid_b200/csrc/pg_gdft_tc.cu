@@ -425,21 +425,21 @@ uint64_t gdft_tc_operand(uint64_t in, int nc) { return gdft_tc_padded(in) / 8 * 
 
 // One CTA per SM at a time: the fewest splits (of at least two tiles) whose
 // last wave is at least 94 % full, else the fullest.
-int gdft_tc_splits(uint64_t out, uint64_t in, int ncp) {
+TcSplit gdft_tc_split(uint64_t out, uint64_t in, int ncp) {
   const uint64_t to = ncp == 8 ? Tc<8>::TO : Tc<16>::TO;
   const uint64_t blocks = (out + to - 1) / to, tiles = gdft_tc_padded(in) / 128, sms = (uint64_t)sm_count();
   const uint64_t most = std::max<uint64_t>(1, std::min<uint64_t>(tiles / 2, 64));
-  uint64_t best = 1;
+  TcSplit best{1, 0};
   double best_eff = 0.0;
   for (uint64_t ns = 1; ns <= most; ++ns) {
     const uint64_t waves = (blocks * ns + sms - 1) / sms;
     // tiles per split are whole: the longest split sets the wave's time
     const uint64_t longest = (tiles + ns - 1) / ns;
     const double eff = (double)(blocks * tiles) / (double)(waves * sms * longest);
-    if (eff > best_eff + 1e-9) { best_eff = eff; best = ns; }
+    if (eff > best_eff + 1e-9) { best_eff = eff; best = {(int)ns, waves * longest}; }
     if (eff >= 0.94) break;
   }
-  return (int)best;
+  return best;
 }
 
 // The operand's last 16 words are the coils' largest entries.

@@ -24,8 +24,13 @@ constexpr uint64_t gdft_tc_padded(uint64_t n) { return (n + 127) / 128 * 128; }
 
 // Coils per tensor pass for C coils (8 or 16).
 int gdft_tc_coils(int C);
-// Splits of the inner sum.
-int gdft_tc_splits(uint64_t out, uint64_t in, int ncp);
+// Splits of the inner sum, and the staged tiles of 128 inputs that the busiest SM
+// then goes through one after another.
+struct TcSplit {
+  int splits;
+  uint64_t steps;
+};
+TcSplit gdft_tc_split(uint64_t out, uint64_t in, int ncp);
 // Words of the packed operand for `in` inputs and nc (8 or 16) coils.
 uint64_t gdft_tc_operand(uint64_t in, int nc);
 // Packs coils [0, nc) of v (S null: v_c[j]; else S_c[j] v[j], one v for all coils).

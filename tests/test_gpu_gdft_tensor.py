@@ -1,5 +1,6 @@
 """SENSE<Gdft> where its sums run on the tensor cores (3 or more coils, at least
-2^25 sample-voxel pairs), against the sums in 64 bits.
+2^25 sample-voxel pairs, and up to 8 coils enough outputs for its CTAs), against
+the sums in 64 bits.
 
 Tolerance 2e-6 relative L2: cos and sin to 2^-21 (the fast intrinsics' bound on
 [-pi, pi]), operands to 2^-23 in two 16-bit parts, sums in FP32; measured
@@ -57,15 +58,35 @@ def _operator(pg, k, t, r, fm, sm):
     return pg.SENSE(pg.Gdft(t.size, N, *k, *r, fm, t), sm.ravel(), t.size, N, nc)
 
 
+def _on_tensor_cores(pg, S, x, y):
+    """Whether the forward and the adjoint run there, by their kernel launches per group of
+    coils: largest entry, packing, sums, finish; the plain kernels have 3 and 2 (groups of 8)."""
+    from powergrid_b200 import _lib
+    nc, out = S.n_data // _samples(S), []
+    for f, v, plain in ((S.forward, x, 3), (S.adjoint, y, 2)):
+        before = _lib.launches()
+        f(v)
+        n = _lib.launches() - before
+        tensor, other = 4 * -(-nc // (8 if nc <= 8 else 16)), plain * -(-nc // 8)
+        assert n in (tensor, other), n
+        out.append(n == tensor)
+    return tuple(out)
+
+
+def _samples(S):
+    return S._keep[0].n_data
+
+
 # outputs and inputs at the edges of tiles (128 inputs, 512 or 1024 outputs),
 # padded and full coil groups, a second group
 @pytest.mark.parametrize("M,shape,nc", [(8192, (16, 16), 3), (8193, (23, 8), 8), (1025, (32, 33), 4), (9999, (24, 6), 9),
-                                        (2100, (26, 24), 16), (3001, (33, 11), 17)])
+                                        (2100, (26, 24), 16), (3001, (33, 11), 17), (1025, (32, 33), 9)])
 def test_tensor_sums_against_64_bits(pg, M, shape, nc):
     k, t, r, fm, sm = _inputs(M, shape, nc)
     g = np.random.default_rng(2)
     N = sm.shape[1]
     assert M * N >= 1 << 25
+    tensor = (M, nc) != (1025, 4)    # few outputs and coils: the plain kernels at the same size
     x = (g.standard_normal(N) + 1j * g.standard_normal(N)).astype(np.complex64)
     y = (g.standard_normal(M * nc) + 1j * g.standard_normal(M * nc)).astype(np.complex64)
     # coils of very different size share no scale
@@ -73,6 +94,7 @@ def test_tensor_sums_against_64_bits(pg, M, shape, nc):
     sm[2] *= np.float32(1e15)
     S = _operator(pg, k, t, r, fm, sm)
     fwd, adj = _both(k, t, r, fm, sm, x, y)
+    assert _on_tensor_cores(pg, S, x, y) == (tensor, tensor)
     got = (S * x).reshape(nc, M)
     for c in range(nc):
         assert rel_l2(got[c], fwd.reshape(nc, M)[c]) <= TOL
@@ -80,7 +102,7 @@ def test_tensor_sums_against_64_bits(pg, M, shape, nc):
 
 
 def test_tensor_sums_with_gradients(pg, oracle):
-    k, t, r, fm, sm = _inputs(4100, (32, 9), 4)
+    k, t, r, fm, sm = _inputs(8190, (32, 9), 4)
     n, N, M = (32, 32, 9), sm.shape[1], t.size
     gd = []
     for off in (1, 32, 1024):   # GdftR2.cpp:62-110
@@ -94,6 +116,7 @@ def test_tensor_sums_with_gradients(pg, oracle):
     x = (g.standard_normal(N) + 1j * g.standard_normal(N)).astype(np.complex64)
     y = (g.standard_normal(M * 4) + 1j * g.standard_normal(M * 4)).astype(np.complex64)
     fwd, adj = _both(k, t, r, fm, sm, x, y, dict(n=n, g=gd))
+    assert _on_tensor_cores(pg, S, x, y) == (True, True)
     assert rel_l2(S * x, fwd) <= 2 * TOL    # plus the three sinc factors in FP32
     assert rel_l2(S / y, adj) <= 2 * TOL
 
@@ -106,16 +129,18 @@ def test_phases_past_the_fixed_point_range(pg):
     x = (g.standard_normal(N) + 1j * g.standard_normal(N)).astype(np.complex64)
     y = (g.standard_normal(M * 3) + 1j * g.standard_normal(M * 3)).astype(np.complex64)
     S = _operator(pg, k, t, r, fm, sm)
+    assert _on_tensor_cores(pg, S, x, y) == (False, False)
     fwd, adj = _both(k, t, r, fm, sm, x, y)
     assert rel_l2(S * x, fwd) <= TOL
     assert rel_l2(S / y, adj) <= TOL
 
 
 def test_non_finite_data_stays_non_finite(pg):
-    k, t, r, fm, sm = _inputs(4200, (32, 9), 4)
+    k, t, r, fm, sm = _inputs(8190, (32, 9), 4)
     M, N = t.size, sm.shape[1]
     S = _operator(pg, k, t, r, fm, sm)
     y = np.ones((4, M), np.complex64)
+    assert _on_tensor_cores(pg, S, np.ones(N, np.complex64), y.ravel()) == (True, True)
     clean = S / y.ravel()
     assert np.isfinite(clean).all()
     for bad in (np.nan, np.inf):
@@ -124,3 +149,20 @@ def test_non_finite_data_stays_non_finite(pg):
         assert not np.isfinite(S / z.ravel()).any()
     zero = S / np.zeros(4 * M, np.complex64)
     assert (zero == 0).all()
+
+
+@pytest.mark.parametrize("M,N,nc,grad,want", [
+    (1100, 30505, 3, 0, (False, False)), (1100, 30505, 8, 0, (False, True)), (1100, 30505, 9, 0, (True, True)),
+    (700, 47935, 5, 0, (False, True)), (8192, 16385, 3, 0, (True, True)), (3472, 15376, 4, 1, (False, False)),
+    (8192, 16385, 4, 1, (True, True)), (400, 83887, 8, 0, (False, False)), (400, 83887, 12, 0, (True, True))])
+def test_few_outputs_or_inputs_stay_on_the_plain_kernels(pg, M, N, nc, grad, want):
+    """Up to 8 coils the tensor kernel's 1024-output CTAs and whole 128-input tiles have to
+    fill the GPU; measured times on both sides are beside the rule (use_tensor)."""
+    g = np.random.default_rng(6)
+    k = ((g.random((3, M)) - 0.5) * 32).astype(np.float32)
+    r = (g.random((3, N)) - 0.5).astype(np.float32)
+    t, fm = np.linspace(0, 10e-3, M).astype(np.float32), (g.random(N) * 300).astype(np.float32)
+    a = (M, N, *k, *r, fm, t)
+    G = pg.GdftR2(*a, N, 1, 1) if grad else pg.Gdft(*a)
+    S = pg.SENSE(G, np.ones(N * nc, np.complex64), M, N, nc)
+    assert _on_tensor_cores(pg, S, np.ones(N, np.complex64), np.ones(M * nc, np.complex64)) == want
