@@ -5,8 +5,8 @@ pg_checks_read returns the first record.
 
 The GPU test runs the checks library in a subprocess (the package loads one
 library per process, chosen by PG_LIBRARY) over the 2-D fused and tiled
-gridding paths (several tiles and coils per item), the 3-D path and a PCG
-solve, and requires every check to pass with results equal to the oracle's
+gridding paths (several tiles and coils per item), the 3-D path (segment windows
+of 1, 2 and 3 segments, several coils) and a PCG solve, and requires every check to pass with results equal to the oracle's
 within the operator tolerance.  No test makes a check fail on the GPU: the
 checks guard indices derived from the binning, which the host validates, so
 a failing check would need a corrupted binning.
@@ -73,6 +73,21 @@ y3 = G3o.forward(x3)
 ef, ea = rel(G3 * x3, y3), rel(G3 / y3, G3o.adjoint(y3))
 rec, en = read()
 out["cases"].append({"case": "3-D Gnufft 16x16x8", "fwd": ef, "adj": ea, "record": rec, "enabled": en})
+# every number of planes per item: segment windows K = 2 (Hanning) and 3 (dense table), odd and even coil counts
+M3, N3 = a.size, n3 * n3 * nz
+fm3 = S.field_map(S.Rng(405), n3, n3, nz, 60.0)
+for L3, typ, nc3 in ((1, 1, 5), (4, 1, 3), (3, 3, 2)):
+    sm3 = S.coil_maps(S.Rng(406), n3, n3, nz, nc3)
+    A3, A3o = G3, G3o
+    if L3 > 1:
+        A3 = pg.TimeSegmentation(G3, fm3, t3, M3, N3, L3, typ, 1)
+        A3o = O.timeseg(G3o, fm3, t3, M3, N3, L3, typ, tables64=typ > 1)
+    S3, S3o = pg.SENSE(A3, sm3, M3, N3, nc3), O.sense(A3o, sm3, M3, N3, nc3)
+    y3 = S3o.forward(x3)
+    ef, ea = rel(S3 * x3, y3), rel(S3 / y3, S3o.adjoint(y3))
+    rec, en = read()
+    out["cases"].append({"case": f"3-D SENSE 16x16x8, L={L3} type {typ}, {nc3} coils", "fwd": ef, "adj": ea,
+                         "record": rec, "enabled": en})
 print("CHECKS " + json.dumps(out))
 """
 

@@ -1,10 +1,12 @@
-"""The oversampled-FFT stage in both of its forms, and gridding edge cases.
+"""The oversampled-FFT stage in all of its forms, and gridding edge cases.
 
-Operators on power-of-two 2N grids (2-D and 3-D) run the library's own
-pruned FFT passes (with the pre/post kernels fused in); PG_CUFFT=1 at
-construction keeps the cuFFT form.  Both must agree with each other and with
-the reference CPU path at the supported grid sizes (in-plane 64 ... 1024, z
-16 ... 128 here), and the gridding must handle the
+Operators with N a multiple of 8 (up to 256, and 512; 2-D and 3-D) run the
+library's own pruned FFT passes with the pre/post kernels fused in; PG_CUFFT=1 at
+construction keeps the cuFFT form, which other N always take.  The own passes
+have forms that the batch's shape chooses: both passes of a small 2-D grid in one
+block, and the sum over an image's grids in one block, in a cluster or through
+images in memory.  Every form must agree with cuFFT's and with the reference CPU
+path at the supported grid sizes, and the gridding must handle the
 trajectory edges the reference's clamped windows define (samples on the
 -N/2 border, a single sample, all samples in one tile).
 
@@ -101,31 +103,53 @@ def test_own_fft_passes_3d_odd_factors(pg, n, nz, L):
         assert rel_l2(own[2] / y, ref[2] / y) <= FORMS_TOL
 
 
-@pytest.mark.parametrize("L,nc", [(1, 1), (4, 3), (8, 8)])
-def test_fused_cluster_passes_equal_separate_passes(pg, L, nc):
-    """The 256x256 grids' one-launch cluster form (rows in each CTA's shared
-    memory, columns over distributed shared memory) against the separate
-    passes: the same transforms in the same order (differences only from the
-    compiler's fma contraction in each kernel), SENSE<TS<Gnufft>> 128^2 with
-    batches of 1, 12 and 64 grids (the last more clusters than fit at once)."""
+def _launches(f, v):
+    from powergrid_b200 import _lib
+    f(v)                                   # binning and workspaces of a first call
+    before = _lib.launches()
+    out = f(v)
+    return out, _lib.launches() - before
+
+
+# The adjoint's launches: spread, both inverse passes, and the sum of the images where
+# they go through memory; 1, 2, 4 and 8 grids per image add up in one block or a
+# cluster, more are shared out over images in memory (12: one each, 64 and 120: several).
+@pytest.mark.parametrize("L,nc,launches", [(1, 1, 3), (2, 1, 3), (4, 1, 3), (8, 1, 3), (2, 3, 3), (4, 3, 4), (8, 8, 4),
+                                           (10, 12, 4)])
+def test_sums_over_an_images_grids_match_cufft(pg, L, nc, launches):
+    """SENSE<TS<Gnufft>> 128^2: every form of the last inverse pass."""
     from powergrid_b200 import synthetic as S
-    _, own = _ts_sense(pg, 128, 8192, L, nc, 77)
-    x = S.image(S.Rng(78), 128 * 128)
-    y = own[2] * x
-    xa = own[2] / y
-    old = os.environ.get("PG_FFT_FUSED")
-    os.environ["PG_FFT_FUSED"] = "0"
-    try:
-        y_sep = own[2] * x
-        xa_sep = own[2] / y
-    finally:
-        if old is None:
-            del os.environ["PG_FFT_FUSED"]
-        else:
-            os.environ["PG_FFT_FUSED"] = old
-    e_f, e_a = rel_l2(y, y_sep), rel_l2(xa, xa_sep)
-    print(f"fused vs separate, L={L}, {nc} coils: forward {e_f:.2e}, adjoint {e_a:.2e}")
-    assert e_f <= 1e-6 and e_a <= 1e-6
+    n = 128
+    _, own = _ts_sense(pg, n, 8192, L, nc, 77)
+    _, ref = _cufft_form(lambda: _ts_sense(pg, n, 8192, L, nc, 77))
+    x = S.image(S.Rng(78), n * n)
+    y, fwd = _launches(own[2].forward, x)
+    xa, adj = _launches(own[2].adjoint, y)
+    assert (fwd, adj) == (3, launches)
+    assert rel_l2(y, ref[2] * x) <= FORMS_TOL and rel_l2(xa, ref[2] / y) <= FORMS_TOL
+
+
+# Up to one grid per SM both passes of a grid run in one block (forward 2 launches with
+# the gather; adjoint 2 with the spread, 3 where the images go through memory); a larger
+# batch runs separate passes.
+@pytest.mark.parametrize("n,L,nc,fwd,adj", [(32, 1, 1, 2, 2), (32, 4, 2, 2, 2), (32, 3, 2, 2, 3), (16, 8, 12, 2, 3),
+                                            (32, 4, 48, 3, 4), (24, 5, 32, 3, 4)])
+def test_small_grids_in_one_block_match_separate_passes(pg, n, L, nc, fwd, adj):
+    """Small 2-D grids: the batch's form against one coil at a time (one block per grid)
+    and against cuFFT."""
+    from powergrid_b200 import synthetic as S
+    arrays, own = _ts_sense(pg, n, 2048, L, nc, 31)
+    _, ref = _cufft_form(lambda: _ts_sense(pg, n, 2048, L, nc, 31))
+    x = S.image(S.Rng(32), n * n)
+    y, lf = _launches(own[2].forward, x)
+    xa, la = _launches(own[2].adjoint, y)
+    assert (lf, la) == (fwd, adj)
+    assert rel_l2(y, ref[2] * x) <= FORMS_TOL and rel_l2(xa, ref[2] / y) <= FORMS_TOL
+    A, sm, M = own[1], arrays[5].reshape(nc, n * n), arrays[0].size
+    one = [A * (c * x).astype(np.complex64) for c in sm]
+    assert rel_l2(y, np.concatenate(one)) <= FORMS_TOL
+    back = sum(np.conj(c) * (A / d).astype(np.complex128) for c, d in zip(sm, y.reshape(nc, M)))
+    assert rel_l2(xa, back) <= FORMS_TOL
 
 
 @pytest.mark.parametrize("n", [128, 256])

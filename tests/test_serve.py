@@ -92,13 +92,13 @@ def test_results_match_direct_api(pg):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [32, 40])
+@pytest.mark.parametrize("n", [32, 40, 42])
 def test_batched_slices_match_per_slice_solves(pg, n):
     """The slices of a request are solved as one stacked operator with per-slice
     inner products and steps; each served slice equals the solve of that slice
     alone through the operator API (reconSolve over its own SENSE<TS<Gnufft>>),
-    with slices that differ in field map, coil maps and data.  n = 32 runs the
-    own FFT passes, n = 40 the cuFFT path; a budget just above one slice's
+    with slices that differ in field map, coil maps and data.  n = 32 and
+    40 run the own FFT passes, n = 42 the cuFFT path; a budget just above one slice's
     footprint splits the request into one job per slice."""
     from powergrid_b200 import synthetic as S
     from powergrid_b200.serve import ReconRequest, Server
