@@ -142,12 +142,6 @@ bool fftpass_supported(const NufftGeom& g) {
   return g.dim == 2 || (g.Gz == 2 * g.Nz && ops_for(g.Gz));
 }
 
-uint64_t fftpass_scratch(const NufftGeom& g, int B) {
-  // 2-D: Nx rows of Gy per grid.  3-D: Nz*Nx rows of Gy, then Nz slabs of Gx*Gy.
-  const uint64_t rows = (uint64_t)g.Nx * g.Nz * g.Gy;
-  return (uint64_t)B * (g.dim == 2 ? rows : rows + (uint64_t)g.Nz * g.Gx * g.Gy);
-}
-
 pg_status fftpass_twiddles(const NufftGeom& g, DevBuf<float2>* tw, cudaStream_t s) {
   std::vector<float2> h;
   twiddle_table(g.Gx, &h);
@@ -213,6 +207,15 @@ static bool one_image_per_grid(const NufftGeom& g, const FftBatch& b, const FftO
   return one_block_per_grid(g, b, op) && (b.cgroup == 0 || (b.c0 % b.cgroup == 0 && b.C % b.cgroup == 0));
 }
 
+// Elements of the half-transformed lines; none where both directions run one block
+// per grid.
+static uint64_t line_scratch(const NufftGeom& g, const FftBatch& b, const FftOps* op) {
+  if (one_image_per_grid(g, b, op)) return 0;
+  // 2-D: Nx rows of Gy per grid.  3-D: Nz*Nx rows of Gy, then Nz slabs of Gx*Gy.
+  const uint64_t rows = (uint64_t)g.Nx * g.Nz * g.Gy;
+  return (uint64_t)b.C * b.L * (g.dim == 2 ? rows : rows + (uint64_t)g.Nz * g.Gx * g.Gy);
+}
+
 static FftRows rows_args(const FftBatch& b, const FftSupport& sup, const float2* W, const float* deapf,
                          const float2* tw, int split, bool cluster = false) {
   return FftRows{b.L, b.C, b.c0, b.cgroup, b.image_stride, b.phase_stride, b.S, b.E, W, deapf, sup.ymask, tw, split,
@@ -220,8 +223,9 @@ static FftRows rows_args(const FftBatch& b, const FftSupport& sup, const float2*
 }
 
 pg_status fftpass_forward(const NufftGeom& g, const FftBatch& b, const FftSupport& sup, const float2* x,
-                          const float2* Wo, const float* deapf, const float2* tw, float2* P, float2* grids,
+                          const float2* Wo, const float* deapf, const float2* tw, float2* scratch, float2* grids,
                           cudaStream_t s) {
+  float2* P = scratch;
   const int B = b.C * b.L;
   if (B > kMaxGridY) return set_error(PG_INVALID_ARG, "fft passes: batch of %d grids", B);
   const FftOps* op = ops_for(g.Gx);
@@ -284,19 +288,23 @@ static InverseSplit inverse_split(const NufftGeom& g, const FftBatch& b, const F
   return {split, split > 1};
 }
 
-uint64_t fftpass_images(const NufftGeom& g, const FftBatch& b) {
-  const InverseSplit is = inverse_split(g, b, ops_for(g.Gx));
-  return is.split == 1 || is.cluster ? 0 : (uint64_t)is.split * batch_images(b) * g.nimg();
+uint64_t fftpass_scratch(const NufftGeom& g, const FftBatch& b) {
+  const FftOps* op = ops_for(g.Gx);
+  const InverseSplit is = inverse_split(g, b, op);
+  const uint64_t images = is.split == 1 || is.cluster ? 0 : (uint64_t)is.split * batch_images(b) * g.nimg();
+  return line_scratch(g, b, op) + images;
 }
 
 pg_status fftpass_adjoint(const NufftGeom& g, const FftBatch& b, const FftSupport& sup, float2* grids, int clear,
-                          const float2* WoH, const float* deapf, const float2* tw, float2* Q, float2* images,
-                          int accumulate, float2* x, cudaStream_t s) {
+                          const float2* WoH, const float* deapf, const float2* tw, float2* scratch, int accumulate,
+                          float2* x, cudaStream_t s) {
   const int B = b.C * b.L;
   if (B > kMaxGridY) return set_error(PG_INVALID_ARG, "fft passes: batch of %d grids", B);
   const uint64_t plane = (uint64_t)g.Gx * g.Gy, rows = (uint64_t)g.Nx * g.Gy, N = g.nimg();
   const int nimages = batch_images(b);
   const FftOps* op = ops_for(g.Gx);
+  float2* Q = scratch;
+  float2* images = scratch + line_scratch(g, b, op);
   const InverseSplit is = inverse_split(g, b, op);
   const bool kept = is.split > 1 && !is.cluster;   // images in memory, added by one more launch
   const FftRows ra = rows_args(b, sup, WoH, deapf, tw, is.split, is.cluster);

@@ -18,8 +18,12 @@ struct FftBatch {
 };
 
 bool fftpass_supported(const NufftGeom& g);
-// Scratch (complex elements) the passes need for a batch of B grids.
-uint64_t fftpass_scratch(const NufftGeom& g, int B);
+// Scratch (complex elements) that either direction may need for a batch: half-
+// transformed lines, then the images of the last inverse pass.  One buffer: an
+// allocation costs some 0.34 ms whatever its size, and a new operator's first calls
+// wait for it (208^2, 12 coils, L = 10, first forward and adjoint: 1.72 ms with the
+// images on their own, 1.38 ms in one).
+uint64_t fftpass_scratch(const NufftGeom& g, const FftBatch& b);
 // Twiddle tables exp(-2 pi i k1 m2 / n) for the in-plane length (and z),
 // made in double precision.
 pg_status fftpass_twiddles(const NufftGeom& g, DevBuf<float2>* tw, cudaStream_t s);
@@ -27,20 +31,17 @@ pg_status fftpass_twiddles(const NufftGeom& g, DevBuf<float2>* tw, cudaStream_t 
 // and segment windows [l0, l0 + K).
 pg_status fftpass_support(const NufftGeom& g, uint64_t M, int L, int K, const uint2* start, const int* l0,
                           FftSupport* out, cudaStream_t s);
-// P: fftpass_scratch elements.  grids: C * L grids out, their supported cells.
+// scratch: fftpass_scratch elements.  grids: C * L grids out, their supported cells.
 pg_status fftpass_forward(const NufftGeom& g, const FftBatch& b, const FftSupport& sup, const float2* x,
-                          const float2* Wo, const float* deapf, const float2* tw, float2* P, float2* grids,
+                          const float2* Wo, const float* deapf, const float2* tw, float2* scratch, float2* grids,
                           cudaStream_t s);
 // Zeroes the supported cells of the batch's 3-D grids.
 pg_status fftpass_clear(const NufftGeom& g, const FftBatch& b, const FftSupport& sup, float2* grids, cudaStream_t s);
-// Elements of the grids' images that fftpass_adjoint keeps in memory (0: none).
-uint64_t fftpass_images(const NufftGeom& g, const FftBatch& b);
 // grids: C * L grids in (after the spread), read in their supported cells;
 // with clear set the first pass zeroes each of them after reading it.
-// Q: fftpass_scratch elements; images: fftpass_images elements;
-// x (+)= the images' sums in a fixed order.
+// scratch: fftpass_scratch elements; x (+)= the images' sums in a fixed order.
 pg_status fftpass_adjoint(const NufftGeom& g, const FftBatch& b, const FftSupport& sup, float2* grids, int clear,
-                          const float2* WoH, const float* deapf, const float2* tw, float2* Q, float2* images,
-                          int accumulate, float2* x, cudaStream_t s);
+                          const float2* WoH, const float* deapf, const float2* tw, float2* scratch, int accumulate,
+                          float2* x, cudaStream_t s);
 
 }  // namespace pg

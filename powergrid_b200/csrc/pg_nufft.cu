@@ -1602,6 +1602,11 @@ static pg_status ensure_adjoint_grids(NufftPlan* p, int B, cudaStream_t s) {
   return PG_OK;
 }
 
+static pg_status ensure_fft_scratch(NufftPlan* p, const FftBatch& b, cudaStream_t s) {
+  const uint64_t n = fftpass_scratch(p->g, b);
+  return n ? grow(p->work->fin, n, s) : PG_OK;
+}
+
 // Forward input grids: the image region is rewritten by every forward, the
 // zero-pad border only here, when the buffer is (re)allocated.  cuFFT's
 // out-of-place C2C transform leaves its input unchanged.
@@ -1918,9 +1923,9 @@ pg_status nufft_forward(NufftPlan* p, const NufftBatch& b, const float2* x, floa
     const int B = nb * L;
     if (p->own_fft) {
       PG_TRY(ensure_workspace(p, B, nullptr, s));
-      PG_TRY(grow(p->work->fin, fftpass_scratch(g, B), s));
-      ProfScope ps("fft_fwd", s);
       const FftBatch fb{nb, L, c0, b.S, b.E, b.cgroup, b.image_stride, b.phase_stride};
+      PG_TRY(ensure_fft_scratch(p, fb, s));
+      ProfScope ps("fft_fwd", s);
       PG_TRY(fftpass_forward(g, fb, *bin->sup, x, b.Wo, p->deapf.p, p->tw2d.p, p->work->fin.p, p->work->grids.p, s));
     } else {
     cufftHandle h;
@@ -2055,13 +2060,11 @@ pg_status nufft_adjoint(NufftPlan* p, const NufftBatch& b, const float2* y, floa
     // passes know which of them began earlier
     const int acc = (b.accumulate || (c0 > 0 && b.cgroup == 0)) ? 1 : 0;
     if (p->own_fft) {
-      PG_TRY(grow(p->work->fin, fftpass_scratch(g, B), s));
       const FftBatch fb{nb, L, c0, b.S, b.E, b.cgroup, b.image_stride, b.phase_stride};
-      const uint64_t images = fftpass_images(g, fb);
-      if (images) PG_TRY(grow(p->work->rimg, images, s));
+      PG_TRY(ensure_fft_scratch(p, fb, s));
       ProfScope ps("fft_adj", s);
-      PG_TRY(fftpass_adjoint(g, fb, *bin->sup, target, self_clear, b.WoH, p->deapf.p, p->tw2d.p, p->work->fin.p,
-                             p->work->rimg.p, acc, x, s));
+      PG_TRY(fftpass_adjoint(g, fb, *bin->sup, target, self_clear, b.WoH, p->deapf.p, p->tw2d.p, p->work->fin.p, acc, x,
+                             s));
       if (self_clear) p->work->agrids_clean = true;   // the first inverse pass leaves the target zero
       continue;
     }

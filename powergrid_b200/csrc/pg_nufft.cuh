@@ -91,9 +91,8 @@ struct NufftWork {
   // stops in between (an error) makes the next one clear it first.
   DevBuf<float2> agrids;
   bool agrids_clean = false;
-  DevBuf<float2> fin;       // forward FFT input; its zero-pad border stays zero
+  DevBuf<float2> fin;       // cuFFT: forward input, its zero-pad border stays zero; own passes: their scratch
   DevBuf<float2> vs;        // adjoint: per-sample segment values in binned order
-  DevBuf<float2> rimg;      // adjoint with the plan's own FFT passes: partial images
   DevBuf<unsigned> queue;   // work-queue words of the persistent spread launches
   DevBuf<char> fft_work;
 };

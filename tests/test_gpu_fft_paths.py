@@ -240,3 +240,24 @@ def test_adjoint_of_zero_data_is_zero(pg):
     G = pg.Gnufft(kx.size, 2.0, n, n, 1, kx, ky, np.zeros_like(kx))
     x = G / np.zeros(kx.size, np.complex64)
     assert np.all(x == 0)
+
+
+def test_first_application_allocates_four_buffers(pg, monkeypatch):
+    """A new operator's first forward and adjoint wait for their workspaces, some 0.34 ms
+    each: the forward's grids, the passes' scratch (with the images of the last inverse
+    pass), the spread's queue and its grids."""
+    import torch
+    from powergrid_b200 import _lib
+    monkeypatch.setenv("PG_AUTOTUNE", "0")
+    _, own = _ts_sense(pg, 104, 4096, 4, 12, 61)
+    A = own[2]
+    x = torch.ones(A.n_image, dtype=torch.complex64, device="cuda")
+    y = torch.ones(A.n_data, dtype=torch.complex64, device="cuda")
+    out = [torch.zeros_like(y), torch.zeros_like(x)]
+    _lib.load().pg_debug_fail_allocation_after(5)
+    try:
+        A.forward(x, out=out[0])
+        A.adjoint(y, out=out[1])
+    finally:
+        _lib.load().pg_debug_fail_allocation_after(0)
+    assert all(bool(o.abs().max() > 0) for o in out)
