@@ -5,10 +5,10 @@
 // Candidates are timed with CUDA events on the operator's own stream and
 // plan (forward + adjoint over a batch of up to 4 coils with synthetic
 // values), in two rounds: tile x bin size with the default coils per block,
-// then the coils per block for the winning binning.  Results are cached per
-// problem shape (dimension, image and sample counts, segments, window, coil
-// batch; the sample count by its power-of-two bucket), so operators of a
-// recurring shape are tuned once per process.  Callers that cannot afford a
+// then the coils per block (2-D: spread and gather, 3-D: gather) for the winning
+// binning.  Results are cached per problem shape (dimension, image and sample
+// counts, segments, window, coil batch; the sample count by its power-of-two
+// bucket), so operators of a recurring shape are tuned once per process.  Callers that cannot afford a
 // search (the request server) only take cached results.
 // PG_AUTOTUNE=0 keeps the defaults (and the PG_TILE2D ... overrides);
 // PG_TUNE_LOG=1 prints each search's choice to stderr.
@@ -148,7 +148,7 @@ pg_status nufft_autotune(NufftPlan* p, int L, int K, const int* l0_host, const f
     float bs = 3e30f, bg = 3e30f;
     int cs_best = best.spread_cc, cg_best = best.gather_cc;
     for (int cc : {1, 2, 4}) {
-      if (cc > Ct) break;
+      if (cc > Ct || g.dim == 3) break;   // the 3-D spread has one form per window width
       p->tune.spread_cc = cc;
       const float ms = time_ms([&] { return nufft_adjoint(p, b, y.p, x.p, s); }, s, kCoilReps);
       if (ms < bs) { bs = ms; cs_best = cc; }

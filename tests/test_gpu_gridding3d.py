@@ -89,3 +89,31 @@ def test_spread_hands_cells_between_lanes(pg, oracle, L, nc):
     want = So.adjoint(y)
     for _ in range(3):
         assert rel_l2(Sg / y, want) <= OP_TOL
+
+
+def test_tuning_skips_what_the_3d_spread_ignores(pg):
+    """The first operator of a shape times its candidates.  The 3-D spread has no choice of
+    coils per item: one adjoint per bin size and repetition, none per number of coils."""
+    from powergrid_b200 import _lib, synthetic as S
+    n, nz, nc = 40, 24, 4
+    kx, ky, kz, t = S.stack_of_spirals(n, nz, 1, 150, 8e-3)
+    M, N = kx.size, n * n * nz
+    sm = S.coil_maps(S.Rng(2), n, n, nz, nc)
+    counts = []
+    for _ in range(2):                     # a search, then its result from the cache
+        G = pg.Gnufft(M, 2.0, n, n, nz, kx, ky, kz)
+        before = _lib.launches()
+        Sg = pg.SENSE(G, sm, M, N, nc)
+        counts.append(_lib.launches() - before)
+    x = S.image(S.Rng(3), N)
+    fwd, adj = [_count(_lib, f, v) for f, v in ((Sg.forward, x), (Sg.adjoint, S.image(S.Rng(4), M * nc)))]
+    builds = 4 * 14                        # at most 14 launches per binning, one per bin size and the default
+    assert counts[0] <= 3 * 3 * (fwd + adj) + 3 * 9 * fwd + builds < 3 * 3 * (fwd + adj) + 3 * 9 * (fwd + adj)
+    assert counts[1] <= 14
+
+
+def _count(_lib, f, v):
+    f(v)
+    before = _lib.launches()
+    f(v)
+    return _lib.launches() - before
