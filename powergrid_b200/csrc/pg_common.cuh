@@ -220,7 +220,6 @@ struct DevBuf {
     if (count) PG_CUDA(cudaMemcpyAsync(p, host, count * sizeof(T), cudaMemcpyHostToDevice, s));
     return PG_OK;
   }
-  size_t bytes() const { return n * sizeof(T); }
 };
 
 // Grow a lazily-sized workspace used on stream s: queued work on s may still

@@ -28,8 +28,8 @@
 // Phase: in units of turns.  q = 1.5 2^20 + kx x + ky y + kz z + (t / 2 pi) FM in
 // double has its unit in the last place at 2^-32, so the low word of q is the
 // fraction of a turn in two's complement: four FP64 fma, no rounding step, no
-// subtraction, no FP64-to-FP32 conversion.  Holds for |phase| < 2^19 turns
-// (checked at plan construction; other plans use pg_gdft.cu's kernels).
+// subtraction, no FP64-to-FP32 conversion.  Holds for |phase| < 2^19 turns; plans
+// are admitted below 2^18 (kTurnLimit), others use pg_gdft.cu's kernels.
 //
 // Split: a CTA is 8 warpgroups (4 with 16 coils) of 128 threads, each with a tile
 // of 128 outputs (one thread and tensor-memory lane per output) and its share of
@@ -38,9 +38,10 @@
 // warpgroup's wait for its matrix product and the latency of its phase chain are
 // covered by the others.
 // What bounds it: the special-function unit (3 conversions or functions per
-// pair at 16 a clock: 11.5 ms at 131072^2 pairs; measured 20.7 ms, from 34.5 ms on
+// pair at 16 a clock: 11.1 ms at 131072^2 pairs; measured 20.8 ms, from 34.8 ms on
 // the plain kernels), the issue slots, and the tensor core's time per
-// instruction.  Forms measured on the way at that size: tf32 operands with 4
+// instruction.  With 8 warpgroups a thread has 64 registers and spills 68 bytes (100
+// with gradients).  Forms measured on the way at that size: tf32 operands with 4
 // warpgroups 24.5 ms, without its matrix instructions 17.7 ms; with 8 warpgroups
 // and steps of 8 inputs 28.9 ms (half as many rows of K per instruction);
 // polynomials in paired FP32 for sine and cosine 30.9 ms (33 instructions per pair).

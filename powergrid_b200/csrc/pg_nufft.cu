@@ -432,8 +432,10 @@ __global__ void __launch_bounds__(128) k_gather(NufftGeom g, TileShape t, const 
 // Taps outside the clamped window weigh 0 and, where they lie outside the grid,
 // are not read.
 // One or two planes are held to 40 registers, six blocks per SM, for the loads'
-// latency.  With 48 and five blocks an operator pair at 96^2 x 16 took 1.01 ms and
-// one at 128^2 x 64 3.14 ms; with 40, 0.99 and 3.06 ms.
+// latency, at the price of 84 and 96 bytes spilled per thread.  With 48 and five blocks
+// an operator pair at 96^2 x 16 took 1.01 ms and one at 128^2 x 64 3.14 ms; with 40, 0.99
+// and 3.06 ms.  More planes take what they need (158 or 172 registers for four, 248 for
+// eight: one block per SM).
 // ---------------------------------------------------------------------------
 constexpr int kGatherRun = 64;    // samples per block: two passes of 32
 
@@ -655,8 +657,8 @@ __global__ void __launch_bounds__(256) k_spread(NufftGeom g, TileShape t, const 
   constexpr int NW = 8;
   const int dy = lane & 7, dx = lane >> 3;
   if (NP > 0) {
-    // Each warp walks a contiguous run of samples.  Samples are in readout
-    // order within a bin, so consecutive ones often share their window start;
+    // Each warp walks a contiguous run of samples.  Samples are ordered by window
+    // (k_order), so consecutive ones often share their window start;
     // a lane then keeps hitting the same two cells, so it sums the run's
     // contributions in registers (paired fp32 fma, fixed order) and issues
     // the shared atomics once per run of equal starts, rounding the run sum
@@ -1340,8 +1342,10 @@ pg_status nufft_plan_create(std::unique_ptr<NufftPlan>* out, uint64_t M, float g
   PG_TRY(p->lut.upload(lut.data(), lut.size(), s));
   p->lut_max = *std::max_element(lut.begin(), lut.end());
   PG_TRY(p->deap.upload(deap.data(), deap.size(), s));
-  // 2N grids with N a multiple of 8 run the pruned, fused FFT passes: 1.5-1.7x
-  // cuFFT's time per operator pair at N = 96 and 208 (pg_fftpass.cu).  Other N
+  // 2N grids with N a multiple of 8 run the pruned, fused FFT passes: an operator
+  // pair takes 0.6-0.7 of its time with cuFFT at N = 96 x 16 and 208 (pg_fftpass.cu), and
+  // of 1304 applications (N = 8 ... 256 and 512, 2-D and 3-D, spirals and random samples,
+  // 1 to 96 grids) none took more than 1.01 of it.  Other N
   // keep cuFFT: the passes' groups of 8 cells and radix-16 pass need 16 | 2N.
   // PG_CUFFT=1 keeps cuFFT everywhere.
   {
@@ -1735,7 +1739,7 @@ static pg_status launch_gather_t(NufftPlan* p, const Binning* bin, const float2*
   return set_error(PG_INVALID_ARG, "forward: unsupported tiling (K=%d)", K);
 }
 
-// 3-D gather launch: CC coils x KP segments per pass, at most 8 planes (16
+// 3-D gather launch: CC <= 4 coils x KP segments per pass, at most 8 planes (16
 // accumulator registers and 8 loads in flight per tap).  The tuner takes one
 // coil at the configurations' sizes: 40 registers, more warps than four coils.
 template <int CC, int KP>
@@ -1752,13 +1756,12 @@ static pg_status launch_gather3d(NufftPlan* p, const Binning* bin, const float2*
   const int K = bin->K;
   const int KP = K <= 1 ? 1 : K <= 2 ? 2 : 4;
   if (K > 3) return set_error(PG_INVALID_ARG, "forward: segment window K=%d too wide", K);
-  int CC = 8 / KP;
+  int CC = std::min(4, 8 / KP);
   while (CC > 1 && (CC >= 2 * nb || CC > p->tune.gather_cc)) CC >>= 1;
   switch (KP * 10 + CC) {
     case 11: return gather3d_launch_one<1, 1>(p, bin, aa, nb, y, dstride, s);
     case 12: return gather3d_launch_one<2, 1>(p, bin, aa, nb, y, dstride, s);
     case 14: return gather3d_launch_one<4, 1>(p, bin, aa, nb, y, dstride, s);
-    case 18: return gather3d_launch_one<8, 1>(p, bin, aa, nb, y, dstride, s);
     case 21: return gather3d_launch_one<1, 2>(p, bin, aa, nb, y, dstride, s);
     case 22: return gather3d_launch_one<2, 2>(p, bin, aa, nb, y, dstride, s);
     case 24: return gather3d_launch_one<4, 2>(p, bin, aa, nb, y, dstride, s);
@@ -1797,14 +1800,12 @@ static pg_status spread_launch_np(NufftPlan* p, const Binning* bin, const Spread
   return PG_OK;
 }
 
-// Planes per block (coils x segments) with an unrolled kernel; others use the
+// Planes per block (coils x segments, K > 2) with an unrolled kernel; others use the
 // runtime-loop instantiation (NP = 0).
 template <int T>
 static pg_status spread_launch_t(NufftPlan* p, const Binning* bin, const SpreadArgs& a, float2* target,
                                  cudaStream_t s) {
   switch (a.cc * bin->K) {
-    case 1: return spread_launch_np<T, 1>(p, bin, a, target, s);
-    case 2: return spread_launch_np<T, 2>(p, bin, a, target, s);
     case 3: return spread_launch_np<T, 3>(p, bin, a, target, s);
     case 4: return spread_launch_np<T, 4>(p, bin, a, target, s);
     case 6: return spread_launch_np<T, 6>(p, bin, a, target, s);

@@ -157,11 +157,6 @@ pg_status GnufftOp::adjoint(const float2* y, float2* x, cudaStream_t s) {
   b.data_stride = plan->M;
   return nufft_adjoint(plan.get(), b, y, x, s);
 }
-uint64_t GnufftOp::resident_bytes() const {
-  if (!plan) return interp ? interp->M * 16 + interp->lut.bytes() : 0;
-  return plan->M * (3 * 4 + 8 + 64 + 4 + 4) + plan->work->grids.bytes() + plan->work->agrids.bytes() +
-         plan->work->fin.bytes();
-}
 
 // ---- Gdft ------------------------------------------------------------------
 pg_status GdftOp::forward(const float2* x, float2* y, cudaStream_t s) {
@@ -307,14 +302,6 @@ pg_status PcSenseTsOp::adjoint(const float2* y, float2* x, cudaStream_t s) {
   }
   return PG_OK;
 }
-uint64_t PcSenseTsOp::resident_bytes() const {
-  uint64_t b = S.bytes() + E.bytes();
-  for (auto& p : plans) b += p->M * 100;
-  if (!plans.empty())
-    b += plans[0]->work->grids.bytes() + plans[0]->work->agrids.bytes() + plans[0]->work->fin.bytes() +
-         plans[0]->work->fft_work.bytes();
-  return b;
-}
 
 // ---- pcSENSE (over Gdft) --------------------------------------------------------
 // fwd column (s + c*Ns) = G_s (x (.) S_c (.) E_s)   (pcSENSE.cpp:113-126)
@@ -335,12 +322,6 @@ pg_status PcSenseOp::adjoint(const float2* y, float2* x, cudaStream_t s) {
     PG_LAUNCH(k_cmul_acc, ceil_div(Ni, 256), 256, 0, s, Ni, tmp.p, E.p + sh * Ni, 0, sh > 0 ? 1 : 0, x);
   }
   return PG_OK;
-}
-uint64_t PcSenseOp::resident_bytes() const {
-  uint64_t b = S.bytes() + E.bytes() + tmp.bytes();
-  for (auto& p : plans) b += p->ks.bytes() + (p->vs.owned ? p->vs.bytes() : 0);
-  if (!plans.empty()) b += plans[0]->work->xin.bytes() + plans[0]->work->part.bytes();
-  return b;
 }
 
 // ---------------------------------------------------------------------------
@@ -384,7 +365,6 @@ pg_status LowRankOp::adjoint(const float2* y, float2* x, cudaStream_t s) {
   return mix_columns(N, (int)Ni, (int)K, stack.p, ca.p, false, x, s);
 }
 
-uint64_t LowRankOp::resident_bytes() const { return cf.bytes() + ca.bytes() + N * Ni * sizeof(float2); }
 
 // The fused gridding stages K segment grids per tile in shared memory: up to
 // 8 in-plane (the forward's register budget), 3 in 3-D (8x8x8 tiles padded

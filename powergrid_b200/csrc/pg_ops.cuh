@@ -34,8 +34,6 @@ struct pg_op_s {
   virtual ~pg_op_s() {}
   virtual pg_status forward(const float2* x, float2* y, cudaStream_t s) = 0;
   virtual pg_status adjoint(const float2* y, float2* x, cudaStream_t s) = 0;
-  // Device bytes held by the operator (admission accounting).
-  virtual uint64_t resident_bytes() const { return 0; }
 };
 
 namespace pg {
@@ -69,7 +67,6 @@ struct GnufftOp : pg_op_s {
   std::unique_ptr<InterpPlan> interp;        // spatial-interpolation tables (Gnufft.cpp:213-337)
   pg_status forward(const float2* x, float2* y, cudaStream_t s) override;
   pg_status adjoint(const float2* y, float2* x, cudaStream_t s) override;
-  uint64_t resident_bytes() const override;
 };
 
 struct GdftOp : pg_op_s {
@@ -106,7 +103,6 @@ struct PcSenseTsOp : pg_op_s {
   DevBuf<float2> S, E;
   pg_status forward(const float2* x, float2* y, cudaStream_t s) override;
   pg_status adjoint(const float2* y, float2* x, cudaStream_t s) override;
-  uint64_t resident_bytes() const override;
 };
 
 // pcSENSE over Gdft (pcSENSE.cpp:40-153): per shot its own Gdft on that shot's
@@ -119,7 +115,6 @@ struct PcSenseOp : pg_op_s {
   DevBuf<float2> tmp;
   pg_status forward(const float2* x, float2* y, cudaStream_t s) override;
   pg_status adjoint(const float2* y, float2* x, cudaStream_t s) override;
-  uint64_t resident_bytes() const override;
 };
 
 // LRobj (lowRank/LRobj.cpp:27-68): x = vec(X), X N x K; forward sends the
@@ -134,7 +129,6 @@ struct LowRankOp : pg_op_s {
   DevBuf<float2> stack;   // N x Nimg image stack
   pg_status forward(const float2* x, float2* y, cudaStream_t s) override;
   pg_status adjoint(const float2* y, float2* x, cudaStream_t s) override;
-  uint64_t resident_bytes() const override;
 };
 
 // The slices of a served request as one operator.  The reference's driver
