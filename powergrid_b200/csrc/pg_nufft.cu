@@ -1243,8 +1243,23 @@ NufftPlan::~NufftPlan() {
   for (auto& kv : ffts) fft_release_plan(g, kv.first, kv.second.first, kv.second.second);
 }
 
-NufftTune NufftTune::defaults(int dim) {
+// Every warp of k_spread3d goes through all samples of its item, so an item where
+// many samples share a tile (the centre of a radial or spiral stack) is the
+// launch's critical path once it holds more than a resident block's average share
+// (three blocks per SM); smaller items cost more tile flushes.  So: that share,
+// rounded down to a power of two, from 64 to 256.  Adjoints of radial stacks in items
+// of 64 / 128 / 256 samples: 32^2 x 16, 8192 samples, one coil 27 / 38 / 59 us (with 256 and
+// the kernel before k_spread3d: 46), 60^2 x 12, 21600 samples 43 / 53 / 73 us (56), 64^2 x 32,
+// 65536 samples 59 / 58 / 73 us (93), there with 4 coils and L = 4 332 / 328 / 325 us.
+int spread3d_items(uint64_t M, int K, int C) {
+  const uint64_t chunks = K == 1 ? (uint64_t)(C + 1) / 2 : (uint64_t)C;   // items per subproblem (launch_spread3d)
+  const uint64_t share = M * chunks / (3ull * (uint64_t)sm_count());
+  return share >= 256 ? 256 : share >= 128 ? 128 : 64;
+}
+
+NufftTune NufftTune::defaults(int dim, uint64_t M) {
   NufftTune t;
+  t.submax3d = spread3d_items(M, 1, 1);
   auto env = [](const char* n, int d) {
     const char* v = getenv(n);
     return (v && *v) ? atoi(v) : d;
@@ -1294,7 +1309,7 @@ pg_status nufft_plan_create(std::unique_ptr<NufftPlan>* out, uint64_t M, float g
                        (unsigned long long)i);
   }
   auto p = std::make_unique<NufftPlan>();
-  p->tune = NufftTune::defaults(nz == 1 ? 2 : 3);
+  p->tune = NufftTune::defaults(nz == 1 ? 2 : 3, M);
   NufftGeom& g = p->g;
   g.dim = (nz == 1) ? 2 : 3;
   g.Nx = nx; g.Ny = ny; g.Nz = nz;

@@ -41,8 +41,11 @@ struct NufftTune {
   int tile2d = 16, tile3d = 8;        // measured best on cfg2 (B200): 16 > 32 > 64
   int submax2d = 256, submax3d = 256;
   int spread_cc = 2, gather_cc = 2;
-  static NufftTune defaults(int dim);
+  static NufftTune defaults(int dim, uint64_t M);
 };
+
+// Most samples of a 3-D item (subproblem) for M samples, windows of K segments and C coils.
+int spread3d_items(uint64_t M, int K, int C);
 
 // Grid cells that a segmentation's taps reach, in groups of 8 adjacent y
 // cells (pg_fftpass.cu).  The own FFT passes leave every other cell alone.

@@ -1,12 +1,12 @@
-// Autotuner for the gridding parameters: tile edge and bin size (samples per
+// Autotuner for the gridding parameters: in 2-D tile edge and bin size (samples per
 // subproblem) of the sample binning, and the coils per block of the spread
-// and gather kernels.
+// and gather kernels; in 3-D, whose bin size follows a rule (spread3d_items), the
+// coils per block of the gather.
 //
 // Candidates are timed with CUDA events on the operator's own stream and
 // plan (forward + adjoint over a batch of up to 4 coils with synthetic
-// values), in two rounds: tile x bin size with the default coils per block,
-// then the coils per block (2-D: spread and gather, 3-D: gather) for the winning
-// binning.  Results are cached per problem shape (dimension, image and sample
+// values), in two rounds: tile x bin size with the default coils per block (2-D),
+// then the coils per block for the winning binning.  Results are cached per problem shape (dimension, image and sample
 // counts, segments, window, coil batch; the sample count by its power-of-two
 // bucket), so operators of a recurring shape are tuned once per process.  Callers that cannot afford a
 // search (the request server) only take cached results.
@@ -115,7 +115,11 @@ pg_status nufft_autotune(NufftPlan* p, int L, int K, const int* l0_host, const f
 
   const NufftTune base = p->tune;
   std::vector<int> tiles = (g.dim == 2) ? std::vector<int>{16, 32} : std::vector<int>{8};
-  const std::vector<int> submaxes = {128, 256, 512};
+  // 3-D items follow a rule: timed on a trajectory without full tiles, where all sizes
+  // are the same binning, noise chose them for every other trajectory of the shape
+  // (items of 512: 96 instead of 54 us on a radial one).
+  const std::vector<int> submaxes =
+      (g.dim == 2) ? std::vector<int>{128, 256, 512} : std::vector<int>{spread3d_items(M, K, Ct)};
   NufftTune best = base;
   std::unique_ptr<Binning> best_bin;
   std::shared_ptr<FftSupport> sup = *bin ? (*bin)->sup : nullptr;
@@ -132,7 +136,7 @@ pg_status nufft_autotune(NufftPlan* p, int L, int K, const int* l0_host, const f
       b.C = Ct;
       b.bin = cand.get();
       b.data_stride = M;
-      const float ms = time_ms([&] {
+      const float ms = g.dim == 3 ? 0.f : time_ms([&] {
         pg_status st = nufft_forward(p, b, x.p, y.p, s);
         return st == PG_OK ? nufft_adjoint(p, b, y.p, x.p, s) : st;
       }, s, 2);

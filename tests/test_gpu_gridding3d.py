@@ -117,3 +117,23 @@ def _count(_lib, f, v):
     before = _lib.launches()
     f(v)
     return _lib.launches() - before
+
+
+@pytest.mark.parametrize("M", [1000, 56800, 56900, 113600, 113700])
+def test_item_sizes_vs_oracle(pg, oracle, M):
+    """Items of 64, 128 and 256 samples (the rule's steps for one coil), full and ragged: half of
+    the samples share the central tiles, as in a radial stack."""
+    from powergrid_b200 import synthetic as S
+    n, nz = 16, 8
+    r = np.random.default_rng(8)
+    k = (r.random((3, M)) - 0.5) * np.array([[n], [n], [nz]]) * 0.99
+    k[:, ::2] *= 0.1
+    kx, ky, kz = k.astype(np.float32)
+    G, ref = pg.Gnufft(M, 2.0, n, n, nz, kx, ky, kz), oracle.gnufft(0, M, n, n, nz, kx, ky, kz)
+    x, y = S.image(S.Rng(9), n * n * nz), S.image(S.Rng(10), M)
+    # one coil is built untuned; SENSE over it takes the items of four coils
+    Sg = pg.SENSE(G, np.ones(4 * x.size, np.complex64), M, x.size, 4)
+    want = ref.adjoint(y)
+    assert rel_l2(G * x, ref.forward(x)) <= OP_TOL
+    assert rel_l2(G / y, want) <= OP_TOL
+    assert rel_l2(Sg / np.tile(y, 4), 4 * want) <= OP_TOL
